@@ -67,24 +67,8 @@ __device__ __forceinline__ float lift_sub(float v, float c, float a, float b)
 	return __fmaf_rn(-c, __fadd_rn(a, b), v);
 }
 
-// Forward lifting over a register window e[0..N); window position j has the
+// Inverse lifting over a register window e[0..N); window position j has the
 // same parity as the signal position it holds. Outputs e[4 .. N-4) are exact.
-template <int N> __device__ __forceinline__ void lift_forward(float (&e)[N])
-{
-#pragma unroll
-	for (int j = 1; j + 1 < N; j += 2)
-		e[j] = lift_add(e[j], kAlpha, e[j - 1], e[j + 1]);
-#pragma unroll
-	for (int j = 2; j + 1 < N; j += 2)
-		e[j] = lift_add(e[j], kBeta, e[j - 1], e[j + 1]);
-#pragma unroll
-	for (int j = 3; j + 1 < N; j += 2)
-		e[j] = lift_add(e[j], kGamma, e[j - 1], e[j + 1]);
-#pragma unroll
-	for (int j = 4; j + 1 < N; j += 2)
-		e[j] = lift_add(e[j], kDelta, e[j - 1], e[j + 1]);
-}
-
 template <int N> __device__ __forceinline__ void lift_inverse(float (&e)[N])
 {
 #pragma unroll
@@ -254,6 +238,27 @@ __device__ __forceinline__ f32x2 f2_fma_rn(f32x2 a, f32x2 b, f32x2 c)
 	f32x2 r;
 	asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
 	return r;
+}
+
+// Forward lifting over a register window of packed pairs (two signals at once,
+// each rounded as alone); window position j has the same parity as the signal
+// position it holds. Outputs e[4 .. N-4) are exact.
+template <int N> __device__ __forceinline__ void lift_forward2(f32x2 (&e)[N])
+{
+	const f32x2 alpha = f2_pack(kAlpha, kAlpha), beta = f2_pack(kBeta, kBeta), gamma = f2_pack(kGamma, kGamma),
+	            delta = f2_pack(kDelta, kDelta);
+#pragma unroll
+	for (int j = 1; j + 1 < N; j += 2)
+		e[j] = f2_fma_rn(alpha, f2_add_rn(e[j - 1], e[j + 1]), e[j]);
+#pragma unroll
+	for (int j = 2; j + 1 < N; j += 2)
+		e[j] = f2_fma_rn(beta, f2_add_rn(e[j - 1], e[j + 1]), e[j]);
+#pragma unroll
+	for (int j = 3; j + 1 < N; j += 2)
+		e[j] = f2_fma_rn(gamma, f2_add_rn(e[j - 1], e[j + 1]), e[j]);
+#pragma unroll
+	for (int j = 4; j + 1 < N; j += 2)
+		e[j] = f2_fma_rn(delta, f2_add_rn(e[j - 1], e[j + 1]), e[j]);
 }
 
 // Thread-block clusters: this CTA's rank, the cluster's CTA count, hardware

@@ -15,14 +15,6 @@ namespace pw
 {
 namespace
 {
-constexpr int kTileIn = 72;  // 64 input samples + 4-sample apron on each side
-// Rows of 76 samples: 16-byte aligned, so the horizontal lifting reads its
-// window as float4 vectors without bank conflicts (76 = 4 * 19, 19 odd), and an
-// interior tile of a level above 0 is one TMA box (72 rows of 76 samples).
-constexpr int kInPitch = 76;
-constexpr uint32_t kInBoxBytes = kTileIn * kInPitch * 4;
-constexpr int kHPitch = 65;
-
 // Reduction scratch of one 128-thread quantiser group (one 32x32 block).
 struct QuantGroupShared
 {
@@ -360,67 +352,117 @@ __device__ __forceinline__ void quant_finish_block(const QuantGroupShared &sh, c
 	}
 }
 
-struct DwtShared
+// Shared memory of one forward-level CTA of kThreads threads and kStripes
+// stripes (DwtSplit below). The input tile is held as pairs of rows (r, r +
+// kPairRows), column by column, so that the horizontal lifting loads packed
+// pairs; after it, rows are plain, and pairs of adjacent columns are packed.
+constexpr int kTileIn = 72;      // 64 input samples + 4-sample apron on each side
+constexpr int kVecs = kTileIn / 4; // vectors of 4 samples per row
+// A row pair's 72 columns as 36 chunks of two pairs, even chunks first: the
+// loader's vector j is chunks 2j and 2j + 1, so lanes of consecutive j write
+// consecutive 16 bytes. Rows of 37 * 16 bytes: lifting lanes (consecutive rows)
+// read without bank conflicts.
+constexpr int kInPitch = 148;
+constexpr int kInOdd = 72;
+constexpr int kHPitch = 68;      // 17 * 16 bytes, as above
+
+template <int kRowsIn> struct DwtSharedT
 {
 	int xidx[kTileIn];
 	int yidx[kTileIn];
-	alignas(128) float in[kTileIn][kInPitch]; // input tile, later the four 32x32 band tiles
-	float h[kTileIn][kHPitch];   // after horizontal lifting: low in 0..31, high in 32..63
+	// The input tile, then (its horizontal lifting done) the four band tiles.
+	union
+	{
+		alignas(16) float in[kRowsIn / 2][kInPitch];
+		alignas(16) float bands[4][kRowsIn == kTileIn ? 32 : 1][kBandPitch];
+	};
+	alignas(16) float h[kRowsIn][kHPitch]; // after horizontal lifting: low in 0..31, high in 32..63
 	QuantGroupShared q[4];
-	float unorm[256];            // unorm8_centered(u) for every byte value
-	uint64_t tile_bar;           // completion of the TMA tile load
 };
 
-__device__ __forceinline__ float unorm8_centered(uint32_t u)
+// Work split of the forward level for a CTA of kThreads threads. Whole tiles
+// of large levels favour few instructions (long lifting segments: 24 samples
+// lifted for 16 kept), stripes and 1024-thread CTAs a short chain.
+template <int kThreads, int kStripes> struct DwtSplit
 {
-	return __fsub_rn(__fdiv_rn(float(u), 255.0f), 0.5f);
-}
-
-// Work split of the forward level for a CTA of kThreads threads. Large levels
-// run many 256-thread CTAs per SM; the small levels, with fewer tiles than
-// SMs, run 1024-thread CTAs that cut every serial phase: shorter lifting
-// windows per thread and all bands quantised in one round with two threads per
-// 4x2 sub-block.
-template <int kThreads> struct DwtSplit
-{
-	static constexpr int kSegPairs = kThreads >= 1024 ? 4 : 8; // output pairs per lifting item
-	static constexpr int kSegs = 32 / kSegPairs;                // items per row / column
-	static constexpr int kWin = 2 * kSegPairs + 8;              // lifting window (4 apron samples each side)
-	static constexpr int kQSplit = kThreads >= 1024 ? 2 : 1;    // threads per 4x2 sub-block in the quantiser
+	static constexpr bool kShort = kThreads >= 1024 || kStripes > 1;
+	static constexpr int kRowsIn = kStripes == 1 ? kTileIn : 64 / kStripes + 8; // input rows loaded and lifted
+	static constexpr int kHPairs = kShort ? 2 : 8; // output pairs per horizontal lifting item
+	static constexpr int kVPairs = kShort ? 2 : 8; // output pairs per vertical lifting item
+	static constexpr int kQSplit = kThreads >= 1024 ? 2 : 1;    // warps per 8x8 row in the quantiser
 	static constexpr int kGroupThreads = 128 * kQSplit;         // threads per quantised 32x32 block
 	static constexpr int kGroups = kThreads / kGroupThreads;    // 32x32 blocks quantised at once
-	static constexpr int kMinBlocks = kThreads >= 1024 ? 1 : (kThreads >= 384 ? 2 : 4); // CTAs per SM to fit
+	static constexpr int kMinBlocks = kThreads >= 1024 ? 1 : 4; // CTAs per SM to fit
 };
+using DwtShared = DwtSharedT<kTileIn>;
 
 // CTA size of the large levels (several CTAs per SM). 384-thread CTAs, which
 // quantise the three high bands of a tile in one round, measured no faster.
 constexpr int kLargeLevelThreads = 256;
 
+// u / 255 - 0.5 and u / 65535 - 0.5, each operation rounded as the division and
+// the subtraction are: the quotient is u * hi + (u * lo rounded), with 1 / n =
+// hi + lo, fused, which equals the rounded quotient for every u in [0, n]
+// (checked for all of them). Two samples at a time; bits holds 2^23 + u.
+__device__ __forceinline__ f32x2 unorm_centered2(uint32_t bits0, uint32_t bits1, bool sample16)
+{
+	const float hi = sample16 ? 0x1.0001p-16f : 0x1.010102p-8f, lo = sample16 ? 0x1.0001p-48f : -0x1.fdfdfep-33f;
+	const f32x2 u = f2_add_rn(f2_pack(__uint_as_float(bits0), __uint_as_float(bits1)), f2_pack(-8388608.0f, -8388608.0f));
+	const f32x2 q = f2_fma_rn(u, f2_pack(hi, hi), f2_mul_rn(u, f2_pack(lo, lo)));
+	return f2_add_rn(q, f2_pack(-0.5f, -0.5f));
+}
+
+// Four samples of a row as raw bits: 8-bit in .x (one byte each), 16-bit in .x
+// and .y, FP32 in all four.
+__device__ __forceinline__ uint32_t pack4_u8(const uint8_t *row, const int4 &x, int xs)
+{
+	const uint32_t a = row[size_t(x.x) * xs], b = row[size_t(x.y) * xs], c = row[size_t(x.z) * xs],
+	               d = row[size_t(x.w) * xs];
+	return __byte_perm(__byte_perm(a, b, 0x0040), __byte_perm(c, d, 0x0040), 0x5410);
+}
+__device__ __forceinline__ uint2 pack4_u16(const uint8_t *row, const int4 &x, int xs)
+{
+	const uint32_t a = *reinterpret_cast<const uint16_t *>(row + size_t(x.x) * xs),
+	               b = *reinterpret_cast<const uint16_t *>(row + size_t(x.y) * xs),
+	               c = *reinterpret_cast<const uint16_t *>(row + size_t(x.z) * xs),
+	               d = *reinterpret_cast<const uint16_t *>(row + size_t(x.w) * xs);
+	return make_uint2(__byte_perm(a, b, 0x5410), __byte_perm(c, d, 0x5410));
+}
+
 // Tile dataflow: waits (bounded) until every tile of the finer level whose LL
-// samples this CTA reads has been stored. The rows and columns read are those
-// of the index tables (mirrored at the edges), so the tiles are the ranges
-// their minimum and maximum fall in: at most 4 x 4 for a whole tile. Called by
-// every thread after the index tables are built; ends with a CTA barrier.
+// samples this CTA reads has been stored: rows and columns of the input window,
+// mirrored at the edges through the index tables, so at most 4 x 4 tiles.
+// Called by every thread (after the index tables of an edge tile are built);
+// ends with a CTA barrier.
 template <int kRowsIn>
-__device__ __forceinline__ void wait_finer_tiles(const DwtShared &sh, const LevelParams &p, const EncodeBuffers &buf,
-                                                 const int comp, const int r0)
+__device__ __forceinline__ void wait_finer_tiles(const int *xidx, const int *yidx, const bool interior, const int x0,
+                                                 const int y0, const LevelParams &p, const EncodeBuffers &buf,
+                                                 const int comp)
 {
 	if (threadIdx.x < 32)
 	{
 		const int lane = threadIdx.x;
-		int ylo = 0x7fffffff, yhi = 0, xlo = 0x7fffffff, xhi = 0;
-		for (int i = lane; i < kRowsIn; i += 32)
+		int ylo = y0, yhi = y0 + kRowsIn - 1, xlo = x0, xhi = x0 + kTileIn - 1;
+		if (!interior)
 		{
-			ylo = min(ylo, sh.yidx[r0 + i]);
-			yhi = max(yhi, sh.yidx[r0 + i]);
+			ylo = xlo = 0x7fffffff;
+			yhi = xhi = 0;
+			for (int i = lane; i < kRowsIn; i += 32)
+			{
+				ylo = min(ylo, yidx[i]);
+				yhi = max(yhi, yidx[i]);
+			}
+			for (int i = lane; i < kTileIn; i += 32)
+			{
+				xlo = min(xlo, xidx[i]);
+				xhi = max(xhi, xidx[i]);
+			}
+			ylo = __reduce_min_sync(0xffffffffu, ylo);
+			yhi = __reduce_max_sync(0xffffffffu, yhi);
+			xlo = __reduce_min_sync(0xffffffffu, xlo);
+			xhi = __reduce_max_sync(0xffffffffu, xhi);
 		}
-		for (int i = lane; i < kTileIn; i += 32)
-		{
-			xlo = min(xlo, sh.xidx[i]);
-			xhi = max(xhi, sh.xidx[i]);
-		}
-		const int ty0 = __reduce_min_sync(0xffffffffu, ylo) >> 5, ty1 = __reduce_max_sync(0xffffffffu, yhi) >> 5;
-		const int tx0 = __reduce_min_sync(0xffffffffu, xlo) >> 5, tx1 = __reduce_max_sync(0xffffffffu, xhi) >> 5;
+		const int ty0 = ylo >> 5, ty1 = yhi >> 5, tx0 = xlo >> 5, tx1 = xhi >> 5;
 		const int w = tx1 - tx0 + 1, n = w * (ty1 - ty0 + 1);
 		const uint32_t *base = buf.tile_done + p.prev_done_offset + comp * p.P.tiles_x * p.P.tiles_y;
 		bool ok = true;
@@ -432,355 +474,13 @@ __device__ __forceinline__ void wait_finer_tiles(const DwtShared &sh, const Leve
 	__syncthreads();
 }
 
-// One forward level for one 32x32 band tile of one component (64x64 input
-// samples): `tile` in row-major tile order, `comp_index` the component among
-// those at this level. Run by every thread of a kThreads-thread CTA. With
-// kStripes > 1 (transform only) the CTA computes one stripe of 32 / kStripes
-// band rows of the tile, one vertical lifting segment: it loads and lifts
-// horizontally only the input rows that segment spans.
-template <int kThreads, int kStripes = 1>
-__device__ __forceinline__ void dwt_forward_body(DwtShared &sh, const LevelParams &p, const PlaneInput &in,
-                                                 const EncodeBuffers &buf, const LevelTileMap *maps, const int fused,
-                                                 const int tile, const int comp_index, const int stripe = 0)
+// Quantises the transmitted bands of a transformed tile in shared memory.
+template <int kThreads>
+__device__ __forceinline__ void quant_tile(DwtShared &sh, const LevelParams &p, const EncodeBuffers &buf, const int fused,
+                                           const int level, const int comp, const int tx, const int ty)
 {
-	using Split = DwtSplit<kThreads>;
-	static_assert(kStripes == 1 || kStripes == Split::kSegs, "a stripe is one vertical lifting segment");
-	// Input rows this CTA loads and lifts horizontally: all 72, or the window of its stripe.
-	constexpr int kRowsIn = kStripes == 1 ? kTileIn : Split::kWin;
-	const int r0 = kStripes == 1 ? 0 : stripe * 2 * Split::kSegPairs;
-	constexpr int kGen = (kRowsIn * kTileIn + kThreads - 1) / kThreads; // gathered loads per thread
-	pdl_trigger();
-	const int level = p.level;
-	const int comp = (level == 0 && !p.chroma444) ? 0 : comp_index;
+	using Split = DwtSplit<kThreads, 1>;
 	const LevelDesc &L = p.L;
-	const int tx = tile % L.tiles_x, ty = tile / L.tiles_x;
-	const bool from_plane = level == 0 || (level == 1 && comp != 0 && !p.chroma444);
-
-	int res_w, res_h, al_w, al_h;
-	if (from_plane)
-	{
-		res_w = p.plane_width[comp];
-		res_h = p.plane_height[comp];
-		al_w = level == 0 ? p.aligned_width : p.aligned_width >> 1;
-		al_h = level == 0 ? p.aligned_height : p.aligned_height >> 1;
-	}
-	else
-	{
-		res_w = al_w = p.P.width;
-		res_h = al_h = p.P.height;
-	}
-
-	// Tile load. A tile whose 72x72 window lies inside the source maps every
-	// sample to itself: an FP32 level above 0 with a tensor map is one TMA box
-	// (barrier and map made ready before the dependency wait); otherwise whole
-	// rows are read with vector loads, all in flight at once. Edge tiles go
-	// through the mirrored index tables in batches of independent loads.
-	const int x0 = tx * 64 - 4, y0 = ty * 64 - 4;
-	const bool interior = x0 >= 0 && y0 >= 0 && x0 + kTileIn <= res_w && y0 + kTileIn <= res_h;
-	const bool use_tma = kStripes == 1 && !from_plane && interior && maps && ((maps->valid >> comp) & 1u) && !p.P.fp16;
-	const CUtensorMap *tmap = use_tma ? &maps->map : nullptr;
-	constexpr int kVecPerRow = kTileIn / 4;     // 18 vectors of 4 samples
-	constexpr int kVecs = kVecPerRow * kRowsIn; // 1296 for a whole tile
-	constexpr int kVecIters = (kVecs + kThreads - 1) / kThreads;
-	const uint8_t *src = comp == 0 ? in.data[0] : (comp == 1 ? in.data[1] : in.data[2]);
-	const int pitch = comp == 0 ? in.pitch[0] : (comp == 1 ? in.pitch[1] : in.pitch[2]);
-	const int xs = comp == 0 ? in.xstride[0] : (comp == 1 ? in.xstride[1] : in.xstride[2]);
-	const bool vec_ok = from_plane && interior && xs == 1 && !in.sample16 &&
-	                    ((reinterpret_cast<uintptr_t>(src) | uintptr_t(pitch)) & 3u) == 0;
-	// An interior tile of an 8-bit input plane is read first, before the index
-	// tables and before the dependency wait: the planes are complete before the
-	// frame's first kernel, so the load latency overlaps the set-up (and, at
-	// level 1, the end of level 0).
-	uint32_t pv[kVecIters];
-	if (vec_ok)
-	{
-#pragma unroll
-		for (int u = 0; u < kVecIters; u++)
-		{
-			const int k = threadIdx.x + u * kThreads;
-			const int ii = k / kVecPerRow, i = r0 + ii, j = k - ii * kVecPerRow;
-			pv[u] = k < kVecs ? __ldg(reinterpret_cast<const uint32_t *>(src + size_t(y0 + i) * pitch + x0) + j) : 0u;
-		}
-	}
-
-	for (int k = threadIdx.x; k < 2 * kTileIn; k += kThreads)
-	{
-		if (k < kTileIn)
-			sh.xidx[k] = fwd_index(tx * 64 - 4 + k, res_w, al_w);
-		else
-			sh.yidx[k - kTileIn] = fwd_index(ty * 64 - 4 + (k - kTileIn), res_h, al_h);
-	}
-	if (from_plane)
-		for (int u = threadIdx.x; u < 256; u += kThreads)
-		{
-			const float f = unorm8_centered(uint32_t(u));
-			sh.unorm[u] = L.stage16 ? round_to_half(f) : f;
-		}
-	if (use_tma && threadIdx.x == 0)
-	{
-		mbarrier_init(&sh.tile_bar, 1);
-		prefetch_tensor_map(tmap);
-	}
-	__syncthreads();
-	if (buf.tile_done)
-	{
-		// Tile dataflow: the input planes are complete before the frame's first
-		// kernel; the finer level's LL is read once the tiles it comes from are.
-		if (!from_plane)
-			wait_finer_tiles<kRowsIn>(sh, p, buf, comp, r0);
-	}
-	else
-		pdl_wait();
-	if (from_plane)
-	{
-		if (in.sample16)
-		{
-			// 16-bit samples (R16_UNORM): u / 65535 - 0.5, gathered through the index tables.
-			for (int base = threadIdx.x; base < kRowsIn * kTileIn; base += kThreads * kGen)
-			{
-				uint32_t v[kGen];
-#pragma unroll
-				for (int u = 0; u < kGen; u++)
-				{
-					const int k = base + u * kThreads;
-					const int ii = k / kTileIn, i = r0 + ii, j = k - ii * kTileIn;
-					v[u] = k < kRowsIn * kTileIn
-					           ? uint32_t(*reinterpret_cast<const uint16_t *>(src + size_t(sh.yidx[i]) * pitch +
-					                                                          size_t(sh.xidx[j]) * xs))
-					           : 0u;
-				}
-#pragma unroll
-				for (int u = 0; u < kGen; u++)
-				{
-					const int k = base + u * kThreads;
-					if (k < kRowsIn * kTileIn)
-					{
-						const int ii = k / kTileIn, i = r0 + ii, j = k - ii * kTileIn;
-						const float f = __fsub_rn(__fdiv_rn(float(v[u]), 65535.0f), 0.5f);
-						sh.in[i][j] = L.stage16 ? round_to_half(f) : f;
-					}
-				}
-			}
-		}
-		else if (vec_ok)
-		{
-#pragma unroll
-			for (int u = 0; u < kVecIters; u++)
-			{
-				const int k = threadIdx.x + u * kThreads;
-				if (k < kVecs)
-				{
-					const int ii = k / kVecPerRow, i = r0 + ii, j = k - ii * kVecPerRow;
-#pragma unroll
-					for (int b = 0; b < 4; b++)
-						sh.in[i][4 * j + b] = sh.unorm[(pv[u] >> (8 * b)) & 0xffu];
-				}
-			}
-		}
-		else
-		{
-			for (int base = threadIdx.x; base < kRowsIn * kTileIn; base += kThreads * kGen)
-			{
-				uint32_t v[kGen];
-#pragma unroll
-				for (int u = 0; u < kGen; u++)
-				{
-					const int k = base + u * kThreads;
-					const int ii = k / kTileIn, i = r0 + ii, j = k - ii * kTileIn;
-					v[u] = k < kRowsIn * kTileIn ? src[size_t(sh.yidx[i]) * pitch + size_t(sh.xidx[j]) * xs] : 0u;
-				}
-#pragma unroll
-				for (int u = 0; u < kGen; u++)
-				{
-					const int k = base + u * kThreads;
-					if (k < kRowsIn * kTileIn)
-					{
-						const int ii = k / kTileIn, i = r0 + ii, j = k - ii * kTileIn;
-						sh.in[i][j] = sh.unorm[v[u] & 0xffu];
-					}
-				}
-			}
-		}
-	}
-	else if (use_tma)
-	{
-		if (threadIdx.x == 0)
-		{
-			if (buf.tile_done)
-				fence_proxy_async_global(); // LL stored by other CTAs, observed through the counters
-			mbarrier_expect_tx(&sh.tile_bar, kInBoxBytes);
-			tma_load_2d(&sh.in[0][0], tmap, x0, maps->row[comp][0] + y0, &sh.tile_bar);
-		}
-		const bool done = mbarrier_wait(&sh.tile_bar, 0, kTmaMaxPolls);
-		if (__syncthreads_or(!done))
-		{
-			// Give up on this tile: record it, and keep the CTA alive (its shared
-			// memory is the copy's destination) for one more bounded wait.
-			if (threadIdx.x == 0)
-				atomicOr(&buf.rc->error, kErrorTileWait);
-			(void)mbarrier_wait(&sh.tile_bar, 0, kTmaMaxPolls);
-			return;
-		}
-	}
-	else
-	{
-		const LevelDesc &P = p.P;
-		const int64_t ll = comp == 0 ? p.prev_ll[0] : (comp == 1 ? p.prev_ll[1] : p.prev_ll[2]);
-		const bool f16 = P.fp16 != 0;
-		if (interior)
-		{
-			float4 v[kVecIters];
-#pragma unroll
-			for (int u = 0; u < kVecIters; u++)
-			{
-				const int k = threadIdx.x + u * kThreads;
-				const int ii = k / kVecPerRow, i = r0 + ii, j = k - ii * kVecPerRow;
-				const int64_t idx = ll + int64_t(y0 + i) * P.pitch + x0 + 4 * j;
-				if (k >= kVecs)
-					v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-				else if (f16)
-				{
-					uint2 hv = __ldcg(reinterpret_cast<const uint2 *>(buf.coef16 + idx));
-					const float2 a = __half22float2(*reinterpret_cast<__half2 *>(&hv.x));
-					const float2 b = __half22float2(*reinterpret_cast<__half2 *>(&hv.y));
-					v[u] = make_float4(a.x, a.y, b.x, b.y);
-				}
-				else
-					v[u] = __ldcg(reinterpret_cast<const float4 *>(buf.coef32 + idx));
-			}
-#pragma unroll
-			for (int u = 0; u < kVecIters; u++)
-			{
-				const int k = threadIdx.x + u * kThreads;
-				if (k < kVecs)
-				{
-					const int ii = k / kVecPerRow, i = r0 + ii, j = k - ii * kVecPerRow;
-					*reinterpret_cast<float4 *>(&sh.in[i][4 * j]) = v[u];
-				}
-			}
-		}
-		else
-		{
-			for (int base = threadIdx.x; base < kRowsIn * kTileIn; base += kThreads * kGen)
-			{
-				float v[kGen];
-#pragma unroll
-				for (int u = 0; u < kGen; u++)
-				{
-					const int k = base + u * kThreads;
-					const int ii = k / kTileIn, i = r0 + ii, j = k - ii * kTileIn;
-					v[u] = k < kRowsIn * kTileIn
-					           ? load_coef(buf.coef32, buf.coef16, f16, ll + int64_t(sh.yidx[i]) * P.pitch + sh.xidx[j])
-					           : 0.0f;
-				}
-#pragma unroll
-				for (int u = 0; u < kGen; u++)
-				{
-					const int k = base + u * kThreads;
-					if (k < kRowsIn * kTileIn)
-					{
-						const int ii = k / kTileIn, i = r0 + ii, j = k - ii * kTileIn;
-						sh.in[i][j] = v[u];
-					}
-				}
-			}
-		}
-	}
-	__syncthreads();
-
-	// Horizontal lifting: 72 rows (the stripe's 24) x kSegs segments of kSegPairs output pairs.
-	constexpr int kSegPairs = Split::kSegPairs, kWin = Split::kWin;
-	for (int item = threadIdx.x; item < kRowsIn * Split::kSegs; item += kThreads)
-	{
-		const int row = r0 + item % kRowsIn, seg = item / kRowsIn;
-		float e[kWin];
-#pragma unroll
-		for (int j = 0; j < kWin; j += 4)
-		{
-			const float4 q = *reinterpret_cast<const float4 *>(&sh.in[row][seg * 2 * kSegPairs + j]);
-			e[j] = q.x;
-			e[j + 1] = q.y;
-			e[j + 2] = q.z;
-			e[j + 3] = q.w;
-		}
-		lift_forward(e);
-#pragma unroll
-		for (int k = 0; k < kSegPairs; k++)
-		{
-			float lo = __fmul_rn(e[4 + 2 * k], kInvK), hi = __fmul_rn(e[5 + 2 * k], kK);
-			if (L.stage16)
-			{
-				lo = round_to_half(lo);
-				hi = round_to_half(hi);
-			}
-			sh.h[row][seg * kSegPairs + k] = lo;
-			sh.h[row][32 + seg * kSegPairs + k] = hi;
-		}
-	}
-	__syncthreads();
-
-	// Vertical lifting: 64 columns x kSegs segments. Columns 0..31 hold the
-	// horizontal low band (-> LL, LH), 32..63 the high band (-> HL, HH).
-	float(*bands)[32][kBandPitch] = reinterpret_cast<float(*)[32][kBandPitch]>(&sh.in[0][0]);
-	constexpr int kVSegs = kStripes == 1 ? Split::kSegs : 1;
-	for (int item = threadIdx.x; item < 64 * kVSegs; item += kThreads)
-	{
-		const int col = item & 63, seg = kStripes == 1 ? item >> 6 : stripe;
-		float e[kWin];
-#pragma unroll
-		for (int j = 0; j < kWin; j++)
-			e[j] = sh.h[seg * 2 * kSegPairs + j][col];
-		lift_forward(e);
-		const int c = col & 31;
-		const int b_low = col < 32 ? 0 : 1, b_high = col < 32 ? 2 : 3;
-		const int gx = tx * 32 + c;
-#pragma unroll
-		for (int k = 0; k < kSegPairs; k++)
-		{
-			const int r = seg * kSegPairs + k;
-			const int gy = ty * 32 + r;
-			float lo = __fmul_rn(e[4 + 2 * k], kInvK);
-			float hi = __fmul_rn(e[5 + 2 * k], kK);
-			if (gx >= L.width || gy >= L.height)
-				lo = hi = 0.0f;
-			else if (L.fp16 || L.stage16)
-			{
-				lo = round_to_half(lo);
-				hi = round_to_half(hi);
-			}
-			bands[b_low][r][c] = lo;
-			bands[b_high][r][c] = hi;
-		}
-	}
-	__syncthreads();
-
-	// Store all four bands (LL feeds the next level): 4 x 32 rows (the stripe's rows) x 8 vectors.
-	constexpr int kBandRows = 32 / kStripes;
-	for (int item = threadIdx.x; item < 4 * kBandRows * 8; item += kThreads)
-	{
-		const int b = item / (kBandRows * 8), r = stripe * kBandRows + (item >> 3) % kBandRows, c4 = (item & 7) * 4;
-		const int64_t idx = p.band[comp][b].offset + int64_t(ty * 32 + r) * L.pitch + tx * 32 + c4;
-		if (L.fp16)
-		{
-			__half2 h0 = __floats2half2_rn(bands[b][r][c4 + 0], bands[b][r][c4 + 1]);
-			__half2 h1 = __floats2half2_rn(bands[b][r][c4 + 2], bands[b][r][c4 + 3]);
-			uint2 u;
-			u.x = *reinterpret_cast<uint32_t *>(&h0);
-			u.y = *reinterpret_cast<uint32_t *>(&h1);
-			*reinterpret_cast<uint2 *>(buf.coef16 + idx) = u;
-		}
-		else
-		{
-			float4 f = make_float4(bands[b][r][c4 + 0], bands[b][r][c4 + 1], bands[b][r][c4 + 2], bands[b][r][c4 + 3]);
-			*reinterpret_cast<float4 *>(buf.coef32 + idx) = f;
-		}
-	}
-
-	if (buf.tile_done)
-		cta_count_done(buf.tile_done + p.done_offset + comp * L.tiles_x * L.tiles_y + tile);
-	if (kStripes > 1 || !fused)
-		return;
-
 	// Quantise the transmitted bands of this tile: HL, LH, HH (+ LL at the last
 	// level), kGroups bands per round. With fused == kFusedSplitTail, a last
 	// round that would leave groups idle (HH after HL and LH in a 256-thread
@@ -795,14 +495,14 @@ __device__ __forceinline__ void dwt_forward_body(DwtShared &sh, const LevelParam
 		split_tail = fused == kFusedSplitTail && (nb % Split::kGroups) != 0;
 	const int rounds = split_tail ? nb / Split::kGroups : (nb + Split::kGroups - 1) / Split::kGroups;
 	for (int bi = grp; bi < min(nb, rounds * Split::kGroups); bi += Split::kGroups)
-		quant_analyze_row<Split::kQSplit>(&bands[first_band + bi][0][0], ly, t >> 7, sh.q[bi], L,
+		quant_analyze_row<Split::kQSplit>(&sh.bands[first_band + bi][0][0], ly, t >> 7, sh.q[bi], L,
 		                                  p.band[comp][first_band + bi], tx, ty, buf);
 	if constexpr (kThreads == kLargeLevelThreads)
 	{
 		if (split_tail)
 		{
 			const int bi = rounds * Split::kGroups;
-			quant_analyze_row<2 * Split::kQSplit>(&bands[first_band + bi][0][0], ly, int(threadIdx.x) >> 7, sh.q[bi],
+			quant_analyze_row<2 * Split::kQSplit>(&sh.bands[first_band + bi][0][0], ly, int(threadIdx.x) >> 7, sh.q[bi],
 			                                      L, p.band[comp][first_band + bi], tx, ty, buf);
 		}
 	}
@@ -825,36 +525,385 @@ __device__ __forceinline__ void dwt_forward_body(DwtShared &sh, const LevelParam
 	}
 }
 
+// One forward level for one 32x32 band tile of one component (64x64 input
+// samples): `tile` in row-major tile order, `comp_index` the component among
+// those at this level. Run by every thread of a kThreads-thread CTA. With
+// kStripes > 1 (transform only) the CTA computes one stripe of 32 / kStripes
+// band rows of the tile: it loads and lifts horizontally only the input rows
+// the stripe spans.
+//
+// Bound by instruction issue (large levels) or by the latency of one load, one
+// store and the barriers between them (small levels), so each pass works on
+// packed pairs of samples (two FP32 operations per instruction), which the
+// shared-memory layouts keep in adjacent registers: rows (r, r + rows / 2) for
+// the horizontal pass, adjacent columns for the vertical one. A loader thread
+// keeps one group of four columns, so the mirrored column indices of an edge
+// tile are read once; samples are converted as they are loaded (no table of
+// 256 values, no tensor-map load whose rows would have to be paired again).
+// Measured against scalar lifting with TMA loads and a table of converted
+// samples: encode of a 720p 4:2:0 frame 37.9 -> 34.9 us, 1080p 49.2 -> 47.5 us,
+// 4K 4:4:4 (1.2 MB) 183 -> 179 us.
+template <int kThreads, int kStripes = 1>
+__device__ __forceinline__ void dwt_forward_body(DwtSharedT<DwtSplit<kThreads, kStripes>::kRowsIn> &sh,
+                                                 const LevelParams &p, const PlaneInput &in, const EncodeBuffers &buf,
+                                                 const int fused, const int tile, const int comp_index,
+                                                 const int stripe = 0)
+{
+	using Split = DwtSplit<kThreads, kStripes>;
+	constexpr int kRowsIn = Split::kRowsIn, kPairRows = kRowsIn / 2;
+	pdl_trigger();
+	const int level = p.level;
+	const int comp = (level == 0 && !p.chroma444) ? 0 : comp_index;
+	const LevelDesc &L = p.L;
+	const int tx = tile % L.tiles_x, ty = tile / L.tiles_x;
+	const bool from_plane = level == 0 || (level == 1 && comp != 0 && !p.chroma444);
+
+	int res_w, res_h, al_w, al_h;
+	if (from_plane)
+	{
+		res_w = p.plane_width[comp];
+		res_h = p.plane_height[comp];
+		al_w = level == 0 ? p.aligned_width : p.aligned_width >> 1;
+		al_h = level == 0 ? p.aligned_height : p.aligned_height >> 1;
+	}
+	else
+	{
+		res_w = al_w = p.P.width;
+		res_h = al_h = p.P.height;
+	}
+
+	// Input window of this CTA. Inside the source every sample maps to itself;
+	// an edge tile goes through the mirrored index tables.
+	const int x0 = tx * 64 - 4, y0 = ty * 64 - 4 + stripe * (64 / kStripes);
+	const bool x_inside = x0 >= 0 && x0 + kTileIn <= res_w, y_inside = y0 >= 0 && y0 + kRowsIn <= res_h;
+	const bool interior = x_inside && y_inside;
+	if (!interior)
+	{
+		for (int k = threadIdx.x; k < kTileIn + kRowsIn; k += kThreads)
+		{
+			if (k < kTileIn)
+				sh.xidx[k] = fwd_index(x0 + k, res_w, al_w);
+			else
+				sh.yidx[k - kTileIn] = fwd_index(y0 + (k - kTileIn), res_h, al_h);
+		}
+		__syncthreads();
+	}
+	// The input planes are complete before the frame's first kernel. With the
+	// tile dataflow a finer level's LL is read once the tiles it comes from are
+	// stored, else after the whole previous grid.
+	if (buf.tile_done)
+	{
+		if (!from_plane)
+			wait_finer_tiles<kRowsIn>(sh.xidx, sh.yidx, interior, x0, y0, p, buf, comp);
+	}
+	else if (!from_plane)
+		pdl_wait();
+
+	// Tile load: a thread takes rows r and r + kPairRows of its four columns,
+	// every load of its iterations in flight at once.
+	constexpr int kLoadRows = kThreads / kVecs; // row pairs per iteration
+	constexpr int kIters = (kPairRows + kLoadRows - 1) / kLoadRows;
+	{
+		const int j = threadIdx.x % kVecs, pr0 = threadIdx.x / kVecs;
+		const bool loader = threadIdx.x < kLoadRows * kVecs;
+		// This thread's four columns are consecutive inside the source, or (edge) gathered.
+		const bool inside = x0 + 4 * j >= 0 && x0 + 4 * j + 4 <= res_w;
+		int4 xi = make_int4(x0 + 4 * j, x0 + 4 * j + 1, x0 + 4 * j + 2, x0 + 4 * j + 3);
+		if (!inside)
+			xi = *reinterpret_cast<const int4 *>(&sh.xidx[4 * j]);
+		auto row_of = [&](int i) { return y_inside ? y0 + i : sh.yidx[i]; };
+		auto put = [&](int pr, const f32x2 (&v)[4]) {
+			float *dst = &sh.in[pr][4 * j];
+			*reinterpret_cast<ulonglong2 *>(dst) = make_ulonglong2(v[0], v[1]);
+			*reinterpret_cast<ulonglong2 *>(dst + kInOdd) = make_ulonglong2(v[2], v[3]);
+		};
+		if (from_plane)
+		{
+			const uint8_t *src = comp == 0 ? in.data[0] : (comp == 1 ? in.data[1] : in.data[2]);
+			const int pitch = comp == 0 ? in.pitch[0] : (comp == 1 ? in.pitch[1] : in.pitch[2]);
+			const int xs = comp == 0 ? in.xstride[0] : (comp == 1 ? in.xstride[1] : in.xstride[2]);
+			const bool wide = in.sample16 != 0;
+			const uintptr_t align = reinterpret_cast<uintptr_t>(src) | uintptr_t(pitch);
+			uint2 raw[kIters][2];
+			if (!wide)
+			{
+				const bool vec = inside && xs == 1 && (align & 3u) == 0;
+				// Unaligned rows: two aligned words around the four bytes, where the
+				// row has bytes on both sides of them.
+				const bool vec_shift = !vec && inside && xs == 1 && x0 + 4 * j >= 4 && x0 + 4 * j + 8 <= res_w;
+#pragma unroll
+				for (int u = 0; u < kIters; u++)
+#pragma unroll
+					for (int h = 0; h < 2; h++)
+					{
+						const int pr = pr0 + u * kLoadRows;
+						raw[u][h].y = 0;
+						if (!loader || pr >= kPairRows)
+							raw[u][h].x = 0;
+						else
+						{
+							const uint8_t *row = src + size_t(row_of(pr + h * kPairRows)) * pitch;
+							if (vec)
+								raw[u][h].x = __ldg(reinterpret_cast<const uint32_t *>(row + xi.x));
+							else if (vec_shift)
+							{
+								const uintptr_t a = reinterpret_cast<uintptr_t>(row + xi.x);
+								const uint32_t *w = reinterpret_cast<const uint32_t *>(a & ~uintptr_t(3));
+								raw[u][h].x = __funnelshift_r(__ldg(w), __ldg(w + 1), 8u * uint32_t(a & 3u));
+							}
+							else
+								raw[u][h].x = pack4_u8(row, xi, xs);
+						}
+					}
+			}
+			else
+			{
+				const bool vec = inside && xs == 2 && (align & 7u) == 0;
+#pragma unroll
+				for (int u = 0; u < kIters; u++)
+#pragma unroll
+					for (int h = 0; h < 2; h++)
+					{
+						const int pr = pr0 + u * kLoadRows;
+						if (!loader || pr >= kPairRows)
+							raw[u][h] = make_uint2(0, 0);
+						else
+						{
+							const uint8_t *row = src + size_t(row_of(pr + h * kPairRows)) * pitch;
+							raw[u][h] = vec ? __ldg(reinterpret_cast<const uint2 *>(row + 2 * xi.x)) : pack4_u16(row, xi, xs);
+						}
+					}
+			}
+#pragma unroll
+			for (int u = 0; u < kIters; u++)
+			{
+				const int pr = pr0 + u * kLoadRows;
+				if (!loader || pr >= kPairRows)
+					continue;
+				f32x2 v[4];
+#pragma unroll
+				for (int b = 0; b < 4; b++)
+				{
+					// Sample b of a row over the exponent of 2^23.
+					uint32_t bits[2];
+#pragma unroll
+					for (int h = 0; h < 2; h++)
+						bits[h] = wide ? __byte_perm(b < 2 ? raw[u][h].x : raw[u][h].y, 0x4B000000u, (b & 1) ? 0x7432 : 0x7410)
+						               : __byte_perm(raw[u][h].x, 0x4B000000u, 0x7440 + b);
+					v[b] = unorm_centered2(bits[0], bits[1], wide);
+					if (L.stage16)
+					{
+						float lo, hi;
+						f2_unpack(v[b], lo, hi);
+						v[b] = f2_pack(round_to_half(lo), round_to_half(hi));
+					}
+				}
+				put(pr, v);
+			}
+			if (!buf.tile_done)
+				pdl_wait(); // before this level's stores
+		}
+		else
+		{
+			const LevelDesc &P = p.P;
+			const int64_t ll = comp == 0 ? p.prev_ll[0] : (comp == 1 ? p.prev_ll[1] : p.prev_ll[2]);
+			const bool f16 = P.fp16 != 0;
+			float4 raw[kIters][2];
+#pragma unroll
+			for (int u = 0; u < kIters; u++)
+#pragma unroll
+				for (int h = 0; h < 2; h++)
+				{
+					const int pr = pr0 + u * kLoadRows;
+					raw[u][h] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+					if (loader && pr < kPairRows)
+					{
+						const int64_t row = ll + int64_t(row_of(pr + h * kPairRows)) * P.pitch;
+						if (!inside)
+							raw[u][h] = make_float4(load_coef(buf.coef32, buf.coef16, f16, row + xi.x),
+							                        load_coef(buf.coef32, buf.coef16, f16, row + xi.y),
+							                        load_coef(buf.coef32, buf.coef16, f16, row + xi.z),
+							                        load_coef(buf.coef32, buf.coef16, f16, row + xi.w));
+						else if (f16)
+						{
+							const uint2 hv = __ldcg(reinterpret_cast<const uint2 *>(buf.coef16 + row + xi.x));
+							const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&hv.x));
+							const float2 b = __half22float2(*reinterpret_cast<const __half2 *>(&hv.y));
+							raw[u][h] = make_float4(a.x, a.y, b.x, b.y);
+						}
+						else
+							raw[u][h] = __ldcg(reinterpret_cast<const float4 *>(buf.coef32 + row + xi.x));
+					}
+				}
+#pragma unroll
+			for (int u = 0; u < kIters; u++)
+			{
+				const int pr = pr0 + u * kLoadRows;
+				if (!loader || pr >= kPairRows)
+					continue;
+				const f32x2 v[4] = {f2_pack(raw[u][0].x, raw[u][1].x), f2_pack(raw[u][0].y, raw[u][1].y),
+				                    f2_pack(raw[u][0].z, raw[u][1].z), f2_pack(raw[u][0].w, raw[u][1].w)};
+				put(pr, v);
+			}
+		}
+	}
+	__syncthreads();
+
+	// Horizontal lifting of row pairs, segments of kHPairs output pairs. Items
+	// start at another warp from tile to tile: they fill half the warps, and
+	// warps of one index share an issue port.
+	{
+		constexpr int kPairs = Split::kHPairs, kSegs = 32 / kPairs, kWin = 2 * kPairs + 8;
+		const int t0 = kStripes == 1 ? (threadIdx.x + 32 * (tile & 3)) & (kThreads - 1) : threadIdx.x;
+		for (int item = t0; item < kPairRows * kSegs; item += kThreads)
+		{
+			const int pr = item % kPairRows, seg = item / kPairRows;
+			f32x2 e[kWin];
+#pragma unroll
+			for (int j = 0; j < kWin; j += 2)
+			{
+				// Pairs j, j + 1 of the window: chunk seg * kPairs + j / 2.
+				const int odd = ((j >> 1) & 1) ? kInOdd : 0;
+				const ulonglong2 v =
+				    *reinterpret_cast<const ulonglong2 *>(&sh.in[pr][odd + (seg * (kPairs / 2) + (j >> 2)) * 4]);
+				e[j] = v.x;
+				e[j + 1] = v.y;
+			}
+			lift_forward2(e);
+			float *const row0 = &sh.h[pr][seg * kPairs], *const row1 = &sh.h[pr + kPairRows][seg * kPairs];
+#pragma unroll
+			for (int k = 0; k < kPairs; k += 2)
+			{
+				float lo0[2], lo1[2], hi0[2], hi1[2]; // [output pair], of rows pr and pr + kPairRows
+#pragma unroll
+				for (int m = 0; m < 2; m++)
+				{
+					float a, b;
+					f2_unpack(e[4 + 2 * (k + m)], a, b);
+					lo0[m] = __fmul_rn(a, kInvK);
+					lo1[m] = __fmul_rn(b, kInvK);
+					f2_unpack(e[5 + 2 * (k + m)], a, b);
+					hi0[m] = __fmul_rn(a, kK);
+					hi1[m] = __fmul_rn(b, kK);
+					if (L.stage16)
+					{
+						lo0[m] = round_to_half(lo0[m]);
+						lo1[m] = round_to_half(lo1[m]);
+						hi0[m] = round_to_half(hi0[m]);
+						hi1[m] = round_to_half(hi1[m]);
+					}
+				}
+				*reinterpret_cast<float2 *>(row0 + k) = make_float2(lo0[0], lo0[1]);
+				*reinterpret_cast<float2 *>(row1 + k) = make_float2(lo1[0], lo1[1]);
+				*reinterpret_cast<float2 *>(row0 + 32 + k) = make_float2(hi0[0], hi0[1]);
+				*reinterpret_cast<float2 *>(row1 + 32 + k) = make_float2(hi1[0], hi1[1]);
+			}
+		}
+	}
+	__syncthreads();
+
+	// Vertical lifting of column pairs. Columns 0..31 hold the horizontal low
+	// band (-> LL, LH), 32..63 the high band (-> HL, HH). Outputs go to storage
+	// and, for the quantiser, to the band tiles; samples beyond the band are
+	// stored as zeros.
+	{
+		constexpr int kPairs = Split::kVPairs, kRows = 32 / kStripes, kSegs = kRows / kPairs, kWin = 2 * kPairs + 8;
+		const bool whole = tx * 32 + 32 <= L.width && ty * 32 + 32 <= L.height;
+		for (int item = threadIdx.x; item < 32 * kSegs; item += kThreads)
+		{
+			const int col = 2 * (item & 31), seg = item >> 5;
+			f32x2 e[kWin];
+#pragma unroll
+			for (int j = 0; j < kWin; j++)
+				e[j] = *reinterpret_cast<const f32x2 *>(&sh.h[seg * 2 * kPairs + j][col]);
+			lift_forward2(e);
+			const int c = col & 31;
+			const int b_low = col < 32 ? 0 : 1;
+			const int gx = tx * 32 + c;
+			const int r0 = stripe * kRows + seg * kPairs;
+			const int64_t at = int64_t(ty * 32 + r0) * L.pitch + gx;
+			const int64_t at_low = p.band[comp][b_low].offset + at, at_high = p.band[comp][b_low + 2].offset + at;
+#pragma unroll
+			for (int k = 0; k < kPairs; k++)
+			{
+				f32x2 lo = f2_mul_rn(e[4 + 2 * k], f2_pack(kInvK, kInvK)), hi = f2_mul_rn(e[5 + 2 * k], f2_pack(kK, kK));
+				if (!whole || L.fp16 || L.stage16)
+				{
+					float a[4];
+					f2_unpack(lo, a[0], a[1]);
+					f2_unpack(hi, a[2], a[3]);
+#pragma unroll
+					for (int i = 0; i < 4; i++)
+					{
+						if (L.fp16 || L.stage16)
+							a[i] = round_to_half(a[i]);
+						if (gx + (i & 1) >= L.width || ty * 32 + r0 + k >= L.height)
+							a[i] = 0.0f;
+					}
+					lo = f2_pack(a[0], a[1]);
+					hi = f2_pack(a[2], a[3]);
+				}
+				if (L.fp16)
+				{
+					float a[4];
+					f2_unpack(lo, a[0], a[1]);
+					f2_unpack(hi, a[2], a[3]);
+					*reinterpret_cast<__half2 *>(buf.coef16 + at_low + k * L.pitch) = __floats2half2_rn(a[0], a[1]);
+					*reinterpret_cast<__half2 *>(buf.coef16 + at_high + k * L.pitch) = __floats2half2_rn(a[2], a[3]);
+				}
+				else
+				{
+					*reinterpret_cast<f32x2 *>(buf.coef32 + at_low + k * L.pitch) = lo;
+					*reinterpret_cast<f32x2 *>(buf.coef32 + at_high + k * L.pitch) = hi;
+				}
+				if (kStripes == 1 && fused)
+				{
+					*reinterpret_cast<f32x2 *>(&sh.bands[b_low][r0 + k][c]) = lo;
+					*reinterpret_cast<f32x2 *>(&sh.bands[b_low + 2][r0 + k][c]) = hi;
+				}
+			}
+		}
+	}
+
+	if (buf.tile_done)
+		cta_count_done(buf.tile_done + p.done_offset + comp * L.tiles_x * L.tiles_y + tile);
+	if constexpr (kStripes == 1)
+	{
+		if (!fused)
+			return;
+		if (!buf.tile_done)
+			__syncthreads();
+		quant_tile<kThreads>(sh, p, buf, fused, level, comp, tx, ty);
+	}
+}
+
 template <int kThreads>
-__global__ void __launch_bounds__(kThreads, DwtSplit<kThreads>::kMinBlocks)
-    dwt_forward_kernel(const LevelParams p, const PlaneInput in, const EncodeBuffers buf, const int fused,
-                       const __grid_constant__ LevelTileMap maps)
+__global__ void __launch_bounds__(kThreads, DwtSplit<kThreads, 1>::kMinBlocks)
+    dwt_forward_kernel(const LevelParams p, const PlaneInput in, const EncodeBuffers buf, const int fused)
 {
 	__shared__ DwtShared sh;
-	dwt_forward_body<kThreads>(sh, p, in, buf, &maps, fused, int(blockIdx.x), int(blockIdx.y));
+	dwt_forward_body<kThreads>(sh, p, in, buf, fused, int(blockIdx.x), int(blockIdx.y));
 }
 
 // Small transform-only levels (fewer tiles than SMs): four 256-thread CTAs per
 // tile, one per stripe of 8 band rows (blockIdx.x = tile * 4 + stripe). Same
 // parameters as dwt_forward_kernel (graph nodes are updated with one argument
-// list); the stripes load with plain vector loads, not tensor maps.
-constexpr int kDwtStripes = DwtSplit<kLargeLevelThreads>::kSegs;
+// list).
+constexpr int kDwtStripes = kDwtStripeCtas;
 __global__ void __launch_bounds__(kLargeLevelThreads, 4)
-    dwt_stripes_kernel(const LevelParams p, const PlaneInput in, const EncodeBuffers buf, const int fused,
-                       const __grid_constant__ LevelTileMap maps)
+    dwt_stripes_kernel(const LevelParams p, const PlaneInput in, const EncodeBuffers buf, const int fused)
 {
 	(void)fused;
-	(void)maps;
-	__shared__ DwtShared sh;
-	dwt_forward_body<kLargeLevelThreads, kDwtStripes>(sh, p, in, buf, nullptr, 0, int(blockIdx.x) / kDwtStripes,
-	                                                  int(blockIdx.y), int(blockIdx.x) % kDwtStripes);
+	__shared__ DwtSharedT<DwtSplit<kLargeLevelThreads, kDwtStripes>::kRowsIn> sh;
+	dwt_forward_body<kLargeLevelThreads, kDwtStripes>(sh, p, in, buf, 0, int(blockIdx.x) / kDwtStripes, int(blockIdx.y),
+	                                                  int(blockIdx.x) % kDwtStripes);
 }
 
 // Batched form: one CTA per (frame, component, tile) of this level.
 template <int kThreads>
-__global__ void __launch_bounds__(kThreads, DwtSplit<kThreads>::kMinBlocks)
+__global__ void __launch_bounds__(kThreads, DwtSplit<kThreads, 1>::kMinBlocks)
     dwt_forward_batch_kernel(const BatchFrame *frames, const BatchFrameIO *io, const uint32_t *cta_map, const int level,
-                             const int fused, const __grid_constant__ BatchTileMaps maps)
+                             const int fused)
 {
 	__shared__ LevelParams s_p;
 	__shared__ PlaneInput s_in;
@@ -867,8 +916,7 @@ __global__ void __launch_bounds__(kThreads, DwtSplit<kThreads>::kMinBlocks)
 	__syncthreads();
 	const int ntiles = s_p.L.tiles_x * s_p.L.tiles_y;
 	__shared__ DwtShared sh;
-	dwt_forward_body<kThreads>(sh, s_p, s_in, s_buf, f < kBatchTileMapFrames ? &maps.frame[f] : nullptr, fused,
-	                           local % ntiles, local / ntiles);
+	dwt_forward_body<kThreads>(sh, s_p, s_in, s_buf, fused, local % ntiles, local / ntiles);
 }
 
 // Quantiser over a pyramid already in storage (the reference's
@@ -1777,7 +1825,7 @@ __device__ __noinline__ void batch_forward_item(int level, int small_level, int 
 {
 	BatchShared &sh = batch_shared();
 	const int per_comp = sh.prm.lp.L.tiles_x * sh.prm.lp.L.tiles_y;
-	dwt_forward_body<kBatchPersistentThreads>(sh.u.dwt, sh.prm.lp, sh.in, sh.eb, nullptr, level < small_level ? 1 : 0,
+	dwt_forward_body<kBatchPersistentThreads>(sh.u.dwt, sh.prm.lp, sh.in, sh.eb, level < small_level ? 1 : 0,
 	                                          local % per_comp, local / per_comp);
 }
 
@@ -1965,27 +2013,24 @@ int forward_fused_mode(const LevelParams &p, bool fused_quant)
 }
 
 void launch_dwt_forward_level(const LevelParams &p, const PlaneInput &in, const EncodeBuffers &buf,
-                              const LevelTileMap *maps, bool fused_quant, bool programmatic, cudaStream_t stream)
+                              bool fused_quant, bool programmatic, cudaStream_t stream)
 {
 	const dim3 grid(p.L.tiles_x * p.L.tiles_y, (p.level == 0 && !p.chroma444) ? 1 : 3);
 	const int f = forward_fused_mode(p, fused_quant);
-	LevelTileMap m = {};
-	if (maps)
-		m = *maps;
 	if (int(grid.x * grid.y) < kSmallLevelTiles && f == 0)
 	{
 		LaunchConfig lc(dim3(grid.x * kDwtStripes, grid.y), dim3(kLargeLevelThreads), stream, programmatic);
-		cudaLaunchKernelEx(&lc.cfg, dwt_stripes_kernel, p, in, buf, f, m);
+		cudaLaunchKernelEx(&lc.cfg, dwt_stripes_kernel, p, in, buf, f);
 	}
 	else if (int(grid.x * grid.y) < kSmallLevelTiles)
 	{
 		LaunchConfig lc(grid, dim3(1024), stream, programmatic);
-		cudaLaunchKernelEx(&lc.cfg, dwt_forward_kernel<1024>, p, in, buf, f, m);
+		cudaLaunchKernelEx(&lc.cfg, dwt_forward_kernel<1024>, p, in, buf, f);
 	}
 	else
 	{
 		LaunchConfig lc(grid, dim3(kLargeLevelThreads), stream, programmatic);
-		cudaLaunchKernelEx(&lc.cfg, dwt_forward_kernel<kLargeLevelThreads>, p, in, buf, f, m);
+		cudaLaunchKernelEx(&lc.cfg, dwt_forward_kernel<kLargeLevelThreads>, p, in, buf, f);
 	}
 }
 
@@ -2095,21 +2140,18 @@ void launch_pack(const BlockParams &p, const EncodeBuffers &buf, cudaStream_t st
 }
 
 void launch_dwt_forward_batch(const BatchFrame *frames, const BatchFrameIO *io, const uint32_t *cta_map, int nctas,
-                              int level, const BatchTileMaps *maps, bool fused_quant, bool large_ctas,
-                              bool programmatic, cudaStream_t stream)
+                              int level, bool fused_quant, bool large_ctas, bool programmatic, cudaStream_t stream)
 {
 	const int f = fused_quant ? 1 : 0;
-	static const BatchTileMaps none = {};
-	const BatchTileMaps &m = maps ? *maps : none;
 	if (large_ctas)
 	{
 		LaunchConfig lc(dim3(nctas), dim3(1024), stream, programmatic);
-		cudaLaunchKernelEx(&lc.cfg, dwt_forward_batch_kernel<1024>, frames, io, cta_map, level, f, m);
+		cudaLaunchKernelEx(&lc.cfg, dwt_forward_batch_kernel<1024>, frames, io, cta_map, level, f);
 	}
 	else
 	{
 		LaunchConfig lc(dim3(nctas), dim3(kLargeLevelThreads), stream, programmatic);
-		cudaLaunchKernelEx(&lc.cfg, dwt_forward_batch_kernel<kLargeLevelThreads>, frames, io, cta_map, level, f, m);
+		cudaLaunchKernelEx(&lc.cfg, dwt_forward_batch_kernel<kLargeLevelThreads>, frames, io, cta_map, level, f);
 	}
 }
 

@@ -653,46 +653,21 @@ bool encode_storage_map(CUtensorMap &map, float *coef32, int64_t storage_elems, 
 	                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Per-level TMA maps of a frame. Forward level l reads its LL input (level
-// l - 1) as boxes of 72 rows x 76 samples; inverse level l reads its four bands
-// as boxes of 36 rows x 40 samples. A component's tiles use the map (valid bit)
-// when its level is FP32, large enough to have interior tiles, and each band it
-// reads starts on a row of the level's pitch; otherwise they use plain loads,
-// as do all tiles when the driver offers no tensor-map encoder. Either table
-// may be null.
-void build_tile_maps(const Geometry &g, const LevelParams (&lp)[kLevels], float *coef32, LevelTileMap *fwd,
-                     LevelTileMap *inv)
+// TMA maps of a frame's inverse levels: level l reads its four bands as boxes
+// of 36 rows x 40 samples. A component's tiles use the map (valid bit) when the
+// level is FP32, large enough to have interior tiles, and each band starts on a
+// row of the level's pitch; otherwise they use plain loads, as do all tiles when
+// the driver offers no tensor-map encoder.
+void build_tile_maps(const Geometry &g, const LevelParams (&lp)[kLevels], float *coef32, LevelTileMap *inv)
 {
 	for (int level = 0; level < kLevels; level++)
-	{
-		if (fwd)
-			fwd[level] = LevelTileMap{};
-		if (inv)
-			inv[level] = LevelTileMap{};
-	}
+		inv[level] = LevelTileMap{};
 	if (!tensor_map_encoder() || !coef32 || g.storage_elems32 <= 0)
 		return;
 	for (int level = 0; level < kLevels; level++)
 	{
 		const LevelParams &p = lp[level];
-		if (fwd && level > 0 && !p.P.fp16 && p.P.pitch >= 76 && p.P.rows >= 72)
-		{
-			LevelTileMap &m = fwd[level];
-			uint32_t valid = 0;
-			for (int comp = 0; comp < kComponents; comp++)
-			{
-				if (level == 1 && comp != 0 && !g.chroma444)
-					continue; // 4:2:0 chroma enters at level 1 from its plane
-				if (p.prev_ll[comp] % p.P.pitch == 0)
-				{
-					m.row[comp][0] = int32_t(p.prev_ll[comp] / p.P.pitch);
-					valid |= 1u << comp;
-				}
-			}
-			if (valid && encode_storage_map(m.map, coef32, g.storage_elems32, p.P.pitch, 76, 72))
-				m.valid = valid;
-		}
-		if (inv && !p.L.fp16 && p.L.pitch >= 40 && p.L.rows >= 36)
+		if (!p.L.fp16 && p.L.pitch >= 40 && p.L.rows >= 36)
 		{
 			LevelTileMap &m = inv[level];
 			uint32_t valid = 0;
@@ -740,7 +715,6 @@ struct pyrowave_encoder_opaque
 	uint32_t *stream_buf = nullptr;
 	uint32_t stream_capacity = 0;
 	uint32_t *jobs_d = nullptr;
-	LevelTileMap in_maps[kLevels] = {}; // TMA maps of the forward transform's LL inputs
 	uint8_t *in_planes[3] = {};
 	int in_pitch[3] = {};
 
@@ -882,7 +856,6 @@ struct pyrowave_encoder_opaque
 			return PYROWAVE_ERROR_OUT_OF_DEVICE_MEMORY;
 		}
 		cudaMemcpy(jobs_d, jobs.data(), jobs.size() * 4, cudaMemcpyHostToDevice);
-		build_tile_maps(g, lp, coef32, in_maps, nullptr);
 		allocated = true;
 		return PYROWAVE_SUCCESS;
 	}
@@ -977,7 +950,7 @@ struct pyrowave_encoder_opaque
 			// waits on the critical path of the transforms.
 			for (int level = 0; level < kLevels; level++)
 			{
-				launch_dwt_forward_level(lp[level], in, b, &in_maps[level], level < small_level, pdl && level > 0, s);
+				launch_dwt_forward_level(lp[level], in, b, level < small_level, pdl && level > 0, s);
 				ok = ok && last_captured_node(s, node_dwt[level]);
 				timing.mark(device, s, dwt_tags[level]);
 			}
@@ -1007,7 +980,7 @@ struct pyrowave_encoder_opaque
 			for (int level = 0; level < kLevels; level++)
 			{
 				int fused = forward_fused_mode(lp[level], level < small_level);
-				ok = ok && set_kernel_args(graph.exec, node_dwt[level], lp[level], pin, b, fused, in_maps[level]);
+				ok = ok && set_kernel_args(graph.exec, node_dwt[level], lp[level], pin, b, fused);
 			}
 			ok = ok && set_kernel_args(graph.exec, node_resolve, rp, b);
 			if (!ok)
@@ -1340,7 +1313,7 @@ struct pyrowave_decoder_opaque
 			cudaMemset(state_d, 0, sizeof(DecodeState));
 		if (ok && cudaEventCreateWithFlags(&decode_done, cudaEventDisableTiming) != cudaSuccess)
 			ok = false;
-		build_tile_maps(g, lp, coef32, nullptr, band_maps);
+		build_tile_maps(g, lp, coef32, band_maps);
 		if (!ok)
 		{
 			release();
@@ -2330,8 +2303,7 @@ pyrowave_result pyrowave_cuda_encoder_transform(pyrowave_encoder encoder, const 
 	const EncodeBuffers b = encoder->buffers();
 	for (int level = 0; level < kLevels; level++)
 	{
-		launch_dwt_forward_level(encoder->lp[level], in, b, &encoder->in_maps[level], false,
-		                         level > 0 && !dev->stage_timing, s);
+		launch_dwt_forward_level(encoder->lp[level], in, b, false, level > 0 && !dev->stage_timing, s);
 		timing.mark(dev, s, tags[level]);
 	}
 	timing.launched(dev);
@@ -2696,8 +2668,7 @@ struct pyrowave_cuda_batch_opaque
 	std::vector<pyrowave_encoder> frame_enc;
 	std::vector<pyrowave_decoder> frame_dec;
 	bool result_frame_graphs = false; // the last call ran in frame-graph mode
-	// Per-level TMA maps of the first kBatchTileMapFrames frames (kernel parameters).
-	std::vector<BatchTileMaps> fwd_maps = std::vector<BatchTileMaps>(kLevels);
+	// Per inverse level, TMA maps of the first kBatchTileMapFrames frames (kernel parameters).
 	std::vector<BatchTileMaps> inv_maps = std::vector<BatchTileMaps>(kLevels);
 
 	BatchShape shape;
@@ -2831,7 +2802,7 @@ struct pyrowave_cuda_batch_opaque
 			if (r.level_n[level] == 0)
 				continue;
 			launch_dwt_forward_batch(frames_d, io_d, maps_d + r.level_off[level], r.level_n[level], level,
-			                         &fwd_maps[level], level < shape.small_level, large(level), pdl, s);
+			                         level < shape.small_level, large(level), pdl, s);
 			pdl = true;
 		}
 		if (r.quant_n > 0)
@@ -3266,13 +3237,10 @@ pyrowave_result pyrowave_cuda_batch_create(pyrowave_device device, const pyrowav
 		di.coef16 = nullptr;
 		if (ok && f < uint32_t(kBatchTileMapFrames))
 		{
-			LevelTileMap fwd[kLevels], inv[kLevels];
-			build_tile_maps(g, fr.lp, eb.coef32, fwd, inv);
+			LevelTileMap inv[kLevels];
+			build_tile_maps(g, fr.lp, eb.coef32, inv);
 			for (int level = 0; level < kLevels; level++)
-			{
-				b->fwd_maps[level].frame[f] = fwd[level];
 				b->inv_maps[level].frame[f] = inv[level];
-			}
 		}
 		fr.block_count = g.block_count_32x32;
 		fr.slices = resolve_slices(g.block_count_32x32, g.blocks_per_subdivision);

@@ -153,7 +153,6 @@ struct DecodeState
 constexpr uint32_t kErrorStreamCapacity = 1u; // the coded frame does not fit the stream buffer
 constexpr uint32_t kErrorWordCount = 2u;      // a packed block's size differs from the rate-control estimate
 constexpr uint32_t kErrorSliceWait = 4u;      // a resolve slice gave up waiting for a preceding slice's total
-constexpr uint32_t kErrorTileWait = 8u;       // a forward-transform tile load did not complete in time
 constexpr uint32_t kErrorLevelWait = 16u;     // a work item gave up waiting for the tiles or items it depends on
 
 // Buffers the encode kernels read and write.
@@ -185,7 +184,7 @@ struct EncodeBuffers
 	uint32_t *tile_done;
 };
 
-// TMA map of one transform level: the frame's FP32 coefficient storage viewed
+// TMA map of one inverse level: the frame's FP32 coefficient storage viewed
 // as rows of one level's pitch, every band of that level starting on a row.
 // Passed as a kernel parameter (grid constant): a map in global memory at an
 // address that earlier held another map can be served stale by the TMA unit's
@@ -194,8 +193,8 @@ struct alignas(64) LevelTileMap
 {
 	CUtensorMap map;
 	uint32_t valid;     // bit c: component c's interior tiles load through the map
-	int32_t row[3][4];  // first row of band b of component c (forward: the LL input, b = 0)
-	// Fault injection for tests (inverse maps only): every tile load that
+	int32_t row[3][4];  // first row of band b of component c
+	// Fault injection for tests: every tile load that
 	// completes is handled as if its bounded wait had run out, which exercises
 	// the error report without stalling the GPU. Set from the environment
 	// variable PYROWAVE_TEST_FAIL_TILE_WAIT=1 when a decoder builds its maps.
@@ -420,8 +419,7 @@ constexpr int kDwtStripeCtas = 4;
 constexpr uint32_t kDataflowWaitSpins = 1u << 20;
 int forward_fused_mode(const LevelParams &p, bool fused_quant);
 void launch_dwt_forward_level(const LevelParams &p, const PlaneInput &in, const EncodeBuffers &buf,
-                              const LevelTileMap *maps, bool fused_quant,
-                              bool programmatic, cudaStream_t stream);
+                              bool fused_quant, bool programmatic, cudaStream_t stream);
 // Quantise and analyse the first nblocks 32x32 blocks (block index order) from storage.
 void launch_quant_pretransformed(const BlockParams &p, const EncodeBuffers &buf, int nblocks, bool programmatic,
                                  cudaStream_t stream);
@@ -472,10 +470,9 @@ void launch_packet_assembly(const PacketParams &pp, cudaStream_t stream);
 
 // Batched launchers: `cta_map` holds one batch_cta() word per CTA.
 // large_ctas selects the 1024-thread variant of a level; `maps` (may be null)
-// holds the level's per-frame TMA maps.
+// holds the inverse level's per-frame TMA maps.
 void launch_dwt_forward_batch(const BatchFrame *frames, const BatchFrameIO *io, const uint32_t *cta_map, int nctas,
-                              int level, const BatchTileMaps *maps, bool fused_quant, bool large_ctas,
-                              bool programmatic, cudaStream_t stream);
+                              int level, bool fused_quant, bool large_ctas, bool programmatic, cudaStream_t stream);
 void launch_quant_blocks_batch(const BatchFrame *frames, const uint32_t *cta_map, int nctas, bool programmatic,
                                cudaStream_t stream);
 void launch_resolve_batch(const BatchFrame *frames, const BatchFrameIO *io, const uint32_t *cta_map, int nctas,
