@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(256, 4) idwt_stripes_kernel(const LevelParams 
                                                               const __grid_constant__ LevelTileMap maps)
 {
 	(void)maps;
-	__shared__ IdwtShared sh;
+	__shared__ IdwtSharedT<IdwtSplit<256, kIdwtStripes>::kOutRows> sh;
 	idwt_body<256, kIdwtStripes>(sh, p, in, out, nullptr, int(blockIdx.x) / kIdwtStripes, int(blockIdx.y),
 	                             int(blockIdx.x) % kIdwtStripes);
 }

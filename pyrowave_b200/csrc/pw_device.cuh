@@ -57,34 +57,6 @@ __device__ __forceinline__ int inv_index_high(int p, int n)
 	return mirrored_repeat(q + 1 >= n ? p + 1 : p, n);
 }
 
-// One lifting update v +/- c * (a + b): a rounded add, then one fused multiply-add.
-__device__ __forceinline__ float lift_add(float v, float c, float a, float b)
-{
-	return __fmaf_rn(c, __fadd_rn(a, b), v);
-}
-__device__ __forceinline__ float lift_sub(float v, float c, float a, float b)
-{
-	return __fmaf_rn(-c, __fadd_rn(a, b), v);
-}
-
-// Inverse lifting over a register window e[0..N); window position j has the
-// same parity as the signal position it holds. Outputs e[4 .. N-4) are exact.
-template <int N> __device__ __forceinline__ void lift_inverse(float (&e)[N])
-{
-#pragma unroll
-	for (int j = 2; j + 1 < N; j += 2)
-		e[j] = lift_sub(e[j], kDelta, e[j - 1], e[j + 1]);
-#pragma unroll
-	for (int j = 3; j + 1 < N; j += 2)
-		e[j] = lift_sub(e[j], kGamma, e[j - 1], e[j + 1]);
-#pragma unroll
-	for (int j = 4; j + 1 < N; j += 2)
-		e[j] = lift_sub(e[j], kBeta, e[j - 1], e[j + 1]);
-#pragma unroll
-	for (int j = 5; j + 1 < N; j += 2)
-		e[j] = lift_sub(e[j], kAlpha, e[j - 1], e[j + 1]);
-}
-
 __device__ __forceinline__ float round_to_half(float v) { return __half2float(__float2half_rn(v)); }
 
 // Programmatic dependent launch (sm_90+ griddepcontrol): let the next kernel
@@ -240,9 +212,10 @@ __device__ __forceinline__ f32x2 f2_fma_rn(f32x2 a, f32x2 b, f32x2 c)
 	return r;
 }
 
-// Forward lifting over a register window of packed pairs (two signals at once,
+// Lifting over a register window of packed pairs (two signals at once,
 // each rounded as alone); window position j has the same parity as the signal
-// position it holds. Outputs e[4 .. N-4) are exact.
+// position it holds. Outputs e[4 .. N-4) are exact. Each update v + c * (a + b)
+// is a rounded sum, then one fused multiply-add; the inverse has -c.
 template <int N> __device__ __forceinline__ void lift_forward2(f32x2 (&e)[N])
 {
 	const f32x2 alpha = f2_pack(kAlpha, kAlpha), beta = f2_pack(kBeta, kBeta), gamma = f2_pack(kGamma, kGamma),
@@ -259,6 +232,24 @@ template <int N> __device__ __forceinline__ void lift_forward2(f32x2 (&e)[N])
 #pragma unroll
 	for (int j = 4; j + 1 < N; j += 2)
 		e[j] = f2_fma_rn(delta, f2_add_rn(e[j - 1], e[j + 1]), e[j]);
+}
+
+template <int N> __device__ __forceinline__ void lift_inverse2(f32x2 (&e)[N])
+{
+	const f32x2 alpha = f2_pack(-kAlpha, -kAlpha), beta = f2_pack(-kBeta, -kBeta), gamma = f2_pack(-kGamma, -kGamma),
+	            delta = f2_pack(-kDelta, -kDelta);
+#pragma unroll
+	for (int j = 2; j + 1 < N; j += 2)
+		e[j] = f2_fma_rn(delta, f2_add_rn(e[j - 1], e[j + 1]), e[j]);
+#pragma unroll
+	for (int j = 3; j + 1 < N; j += 2)
+		e[j] = f2_fma_rn(gamma, f2_add_rn(e[j - 1], e[j + 1]), e[j]);
+#pragma unroll
+	for (int j = 4; j + 1 < N; j += 2)
+		e[j] = f2_fma_rn(beta, f2_add_rn(e[j - 1], e[j + 1]), e[j]);
+#pragma unroll
+	for (int j = 5; j + 1 < N; j += 2)
+		e[j] = f2_fma_rn(alpha, f2_add_rn(e[j - 1], e[j + 1]), e[j]);
 }
 
 // Thread-block clusters: this CTA's rank, the cluster's CTA count, hardware
