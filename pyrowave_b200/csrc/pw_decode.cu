@@ -13,19 +13,18 @@ namespace pw
 {
 namespace
 {
-// One 32x32 block per 64-thread CTA, two sub-blocks per thread: twice the
-// blocks resident per SM of 128-thread CTAs (a 1080p frame's 3261 blocks in
-// one wave).
+// Two 32x32 blocks per CTA: a 1080p frame's 3261 blocks are resident in one wave.
 constexpr int kDequantThreads = 64;
-__global__ void __launch_bounds__(kDequantThreads) dequant_kernel(const BlockParams p, const DecodeInput in, const int first)
+__global__ void __launch_bounds__(kDequantThreads) dequant_kernel(const BlockParams p, const DecodeInput in)
 {
-	__shared__ DequantShared sh;
-	// Only the launch that starts at block 0 clears the decode's error word.
-	dequant_body<128 / kDequantThreads>(sh, p, in, first + int(blockIdx.x), blockIdx.x == 0 && first == 0, 1);
+	__shared__ DequantShared sh[kDequantThreads / 32];
+	const int warp = int(threadIdx.x) >> 5, blk = int(blockIdx.x) * (kDequantThreads / 32) + warp;
+	if (blk < p.block_count_32x32)
+		dequant_body(sh[warp], p, in, blk, blk == 0);
 }
 
-// Batched form: one CTA per (frame, block), decoding the frame's own bitstream.
-__global__ void __launch_bounds__(128) dequant_batch_kernel(const BatchFrame *frames, const uint32_t *cta_map)
+// Batched form: one 32-thread CTA per (frame, block), decoding the frame's own bitstream.
+__global__ void __launch_bounds__(32) dequant_batch_kernel(const BatchFrame *frames, const uint32_t *cta_map)
 {
 	__shared__ BlockParams s_p;
 	__shared__ DecodeInput s_in;
@@ -35,7 +34,7 @@ __global__ void __launch_bounds__(128) dequant_batch_kernel(const BatchFrame *fr
 	load_params(s_in, frames[f].di);
 	__syncthreads();
 	__shared__ DequantShared sh;
-	dequant_body(sh, s_p, s_in, local, local == 0, 1);
+	dequant_body(sh, s_p, s_in, local, local == 0);
 }
 
 // 256-thread CTAs: three per SM (80 registers) for levels of about one wave,
@@ -116,11 +115,11 @@ __global__ void pyramid_io_kernel(const BlockParams p, float *canonical, float *
 }
 } // namespace
 
-void launch_dequant(const BlockParams &p, const DecodeInput &in, int first, int count, bool programmatic,
-                    cudaStream_t stream)
+void launch_dequant(const BlockParams &p, const DecodeInput &in, bool programmatic, cudaStream_t stream)
 {
-	LaunchConfig lc(dim3(count), dim3(kDequantThreads), stream, programmatic);
-	cudaLaunchKernelEx(&lc.cfg, dequant_kernel, p, in, first);
+	constexpr int kBlocks = kDequantThreads / 32;
+	LaunchConfig lc(dim3((p.block_count_32x32 + kBlocks - 1) / kBlocks), dim3(kDequantThreads), stream, programmatic);
+	cudaLaunchKernelEx(&lc.cfg, dequant_kernel, p, in);
 }
 
 // SMs of the current device (queried once).
@@ -177,7 +176,7 @@ void launch_pyramid_io(const BlockParams &p, float *canonical, float *coef32, __
 void launch_dequant_batch(const BatchFrame *frames, const uint32_t *cta_map, int nctas, bool programmatic,
                           cudaStream_t stream)
 {
-	LaunchConfig lc(dim3(nctas), dim3(128), stream, programmatic);
+	LaunchConfig lc(dim3(nctas), dim3(32), stream, programmatic);
 	cudaLaunchKernelEx(&lc.cfg, dequant_batch_kernel, frames, cta_map);
 }
 
@@ -281,7 +280,7 @@ extern "C" pyrowave_result pyrowave_cuda_decode_blocks_static(int width, int hei
 	in.coef32 = scratch;
 	in.coef16 = nullptr; // every level is FP32 here
 	const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-	launch_dequant(make_block_params(g), in, 0, g.block_count_32x32, false, s);
+	launch_dequant(make_block_params(g), in, false, s);
 	for (int level = kLevels - 1; level >= 0; level--)
 		launch_idwt_level(make_level_params(g, level), in, out, nullptr, true, s);
 	return cudaGetLastError() == cudaSuccess ? PYROWAVE_SUCCESS : PYROWAVE_ERROR_GENERIC;

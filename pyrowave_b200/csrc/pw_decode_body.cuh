@@ -22,62 +22,58 @@ struct PayloadReader
 	const uint32_t *words;
 	uint32_t nwords;
 	__device__ __forceinline__ uint32_t w32(uint32_t i) const { return i < nwords ? __ldcg(words + i) : 0u; }
-	__device__ __forceinline__ uint32_t u8(uint32_t i) const { return (w32(i >> 2) >> (8u * (i & 3u))) & 0xffu; }
-	__device__ __forceinline__ uint32_t u16(uint32_t i) const { return (w32(i >> 1) >> (16u * (i & 1u))) & 0xffffu; }
 };
 
-// A block's words staged in shared memory: words [base, base + count) of the
-// payload come from `s`, anything else from the bounds-checked global reader,
-// so reads of a malformed block behave exactly as with PayloadReader alone.
-struct StagedReader
+// A block's words staged in shared memory, addressed from the block's first
+// word. With kChecked, words beyond `count` come from the bounds-checked global
+// reader (a malformed block reads on into what follows it, never out of
+// bounds); without, the caller has made sure that every word read is staged.
+template <bool kChecked> struct BlockReader
 {
 	const uint32_t *s;
-	uint32_t base, count;
+	uint32_t off, count;
 	PayloadReader g;
-	__device__ __forceinline__ uint32_t w32(uint32_t i) const
+	__device__ __forceinline__ uint32_t w32(uint32_t r) const
 	{
-		const uint32_t r = i - base;
-		return r < count ? s[r] : g.w32(i);
+		if constexpr (kChecked)
+			return r < count ? s[r] : g.w32(off + r);
+		else
+			return s[r];
 	}
-	__device__ __forceinline__ uint32_t u8(uint32_t i) const { return (w32(i >> 2) >> (8u * (i & 3u))) & 0xffu; }
-	__device__ __forceinline__ uint32_t u16(uint32_t i) const { return (w32(i >> 1) >> (16u * (i & 1u))) & 0xffffu; }
+	__device__ __forceinline__ uint32_t u8(uint32_t r) const
+	{
+		if constexpr (kChecked)
+			return (w32(r >> 2) >> (8u * (r & 3u))) & 0xffu;
+		else
+			return reinterpret_cast<const uint8_t *>(s)[r];
+	}
+	__device__ __forceinline__ uint32_t u16(uint32_t r) const
+	{
+		if constexpr (kChecked)
+			return (w32(r >> 1) >> (16u * (r & 1u))) & 0xffffu;
+		else
+			return reinterpret_cast<const uint16_t *>(s)[r];
+	}
 };
 
 constexpr uint32_t kSpeculativeWords = 128; // staged with the header when the block size is not yet known
 
-// s[i] = payload word off + i for i in [begin, end), by kThreads threads with
-// up to eight loads per thread in flight together.
-template <int kThreads = 128>
+// s[i] = payload word off + i for i in [begin, end), by one warp with up to
+// eight loads per lane in flight together.
 __device__ __forceinline__ void stage_words(uint32_t *s, const PayloadReader &g, uint32_t off, uint32_t begin,
-                                            uint32_t end, int t)
+                                            uint32_t end)
 {
-	for (uint32_t base = begin + uint32_t(t); base < end; base += kThreads * 8)
+	for (uint32_t base = begin + (threadIdx.x & 31); base < end; base += 32 * 8)
 	{
 		uint32_t v[8];
 #pragma unroll
 		for (int u = 0; u < 8; u++)
-		{
-			const uint32_t i = base + uint32_t(kThreads) * u;
-			v[u] = i < end ? g.w32(off + i) : 0u;
-		}
+			v[u] = base + 32u * u < end ? g.w32(off + base + 32u * u) : 0u;
 #pragma unroll
 		for (int u = 0; u < 8; u++)
-		{
-			const uint32_t i = base + uint32_t(kThreads) * u;
-			if (i < end)
-				s[i] = v[u];
-		}
+			if (base + 32u * u < end)
+				s[base + 32u * u] = v[u];
 	}
-}
-
-// The barrier of a block's thread group: hardware barrier `bar` of 128
-// threads, or the whole CTA when a CTA holds one smaller group.
-template <int kSubs> __device__ __forceinline__ void block_sync(int bar)
-{
-	if constexpr (kSubs == 1)
-		group_sync(bar);
-	else
-		__syncthreads();
 }
 
 __device__ __forceinline__ void store_coef(float *c32, __half *c16, bool fp16, int64_t idx, float v)
@@ -88,49 +84,174 @@ __device__ __forceinline__ void store_coef(float *c32, __half *c16, bool fp16, i
 		c32[idx] = v;
 }
 
-// One 32x32 block per thread group; thread = one 4x2 sub-block (the
-// reference's mapping, wavelet_dequant.comp:222-238), or kSubs sub-blocks two
-// 8x8 rows apart. The group with `clear_error` set clears the decode's error
-// word: every inverse level runs after the dequantiser has completed, so the
-// clear precedes any error report.
+// A warp's staging area: the block's words and room for the reads of whole
+// words just past them.
 struct DequantShared
 {
-	uint32_t s_words[kMaxBlockWords];
-	uint32_t s_plane_off[16];
-	uint32_t s_sign_base;
-	uint32_t s_sig[4];
+	uint32_t words[kMaxBlockWords + 4];
 };
 
-// One 32x32 block on a group of 128 / kSubs threads: with kSubs = 1 the group
-// is threadIdx.x & 127, synchronised with hardware barrier `bar`; with kSubs =
-// 2 the whole 64-thread CTA, each thread decoding the sub-blocks of 8x8 rows
-// ly and ly + 2.
-template <int kSubs = 1>
-__device__ __forceinline__ void dequant_body(DequantShared &sh, const BlockParams &p, const DecodeInput &in,
-                                             const int blk, const bool clear_error, const int bar)
+// Magnitudes and signs of one staged block (see dequant_body), its four rows'
+// sub-blocks stored as coefficients.
+template <bool kChecked>
+__device__ __forceinline__ void dequant_block(const BlockReader<kChecked> &rd, const uint32_t ballot,
+                                              const uint32_t header, const uint32_t first_byte, uint32_t sign_bit,
+                                              const float quant, const DecodeInput &in, const bool f16, const int64_t at,
+                                              const int pitch)
 {
-	static_assert(kSubs == 1 || kSubs == 2, "one or two sub-blocks per thread");
-	constexpr int kGroup = 128 / kSubs;
-	constexpr int kRowStep = 4 / kSubs;
-	uint32_t *const s_words = sh.s_words;
-	uint32_t *const s_plane_off = sh.s_plane_off;
-	uint32_t &s_sign_base = sh.s_sign_base;
-	uint32_t *const s_sig = sh.s_sig;
+	const unsigned full = 0xffffffffu;
+	const int lane = threadIdx.x & 31, sub = lane & 7, lx = lane >> 3;
+	float v[4][8];
+	uint32_t sig4 = 0;
+#pragma unroll
+	for (int h = 0; h < 4; h++)
+	{
+#pragma unroll
+		for (int i = 0; i < 8; i++)
+			v[h][i] = 0.0f;
+		if (((ballot >> (4 * h)) & 0xfu) == 0)
+			continue; // no coded 8x8 in the row
+		// Lane grp of the header pass holds 8x8 grp: code word, Q bits, scale.
+		const int grp = 4 * h + lx;
+		const uint32_t cw = __shfl_sync(full, header, grp);
+		uint32_t byte = __shfl_sync(full, first_byte, grp);
+		const uint32_t qb = (cw >> 16) & 0xfu;
+		const uint32_t before = (1u << (2 * sub)) - 1u;
+		byte += uint32_t(plane_code_sum(cw & before, 0)) + qb * uint32_t(sub);
+		const uint32_t planes = (cw & 0xffffu) != 0 ? qb + ((cw >> (2 * sub)) & 3u) : 0u;
+		const float scale = __fmul_rn(quant, decode_quant_scale((cw >> 20) & 0xfu));
+		uint32_t sig = 0;
+		if (__reduce_max_sync(full, planes) <= 8)
+		{
+			// The sub-block's plane bytes (most significant first) as one 64-bit
+			// window, turned round and moved down so that byte k is plane k: the
+			// rows of an 8x8 bit matrix; transposed, byte i is coefficient i.
+			unsigned long long m = 0;
+			if (planes != 0)
+			{
+				const uint32_t w = byte >> 2, sh = 8u * (byte & 3u);
+				const uint32_t a = rd.w32(w), b = rd.w32(w + 1), c = rd.w32(w + 2);
+				const uint32_t lo = __funnelshift_r(a, b, sh), hi = __funnelshift_r(b, c, sh);
+				m = ((unsigned long long)(__byte_perm(lo, 0, 0x0123)) << 32 | __byte_perm(hi, 0, 0x0123)) >>
+				    (8u * (8u - planes));
+			}
+			sig = uint32_t(m) | uint32_t(m >> 32);
+			sig |= sig >> 16;
+			sig = (sig | (sig >> 8)) & 0xffu;
+			m = transpose8x8(m);
+#pragma unroll
+			for (int i = 0; i < 8; i += 2)
+			{
+				// Magnitude + 0.5: the byte over the exponent of 2^23, minus 2^23 - 0.5.
+				const uint32_t w = i < 4 ? uint32_t(m) : uint32_t(m >> 32);
+				const f32x2 f = f2_add_rn(f2_pack(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440 + (i & 3))),
+				                                  __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7441 + (i & 3)))),
+				                          f2_pack(-8388607.5f, -8388607.5f));
+				f2_unpack(f, v[h][i], v[h][i + 1]);
+			}
+		}
+		else
+		{
+			// More than eight planes somewhere in the row (more than sixteen only
+			// in a malformed one): plane by plane.
+			uint32_t dec[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+			for (int pl = int(planes) - 1; pl >= 0; pl--)
+			{
+				const uint32_t bits = rd.u8(byte++);
+#pragma unroll
+				for (int i = 0; i < 8; i++)
+					dec[i] |= ((bits >> i) & 1u) << pl;
+			}
+#pragma unroll
+			for (int i = 0; i < 8; i++)
+			{
+				sig |= dec[i] != 0 ? 1u << i : 0u;
+				v[h][i] = __fadd_rn(float(dec[i]), 0.5f);
+			}
+		}
+		sig4 |= sig << (8 * h);
+#pragma unroll
+		for (int i = 0; i < 8; i++)
+			v[h][i] = __fmul_rn(v[h][i], scale);
+	}
+
+	// Sign bits: position = number of significant coefficients before this one
+	// (in sub-block order: 8x8 rows, then the 32 sub-blocks of a row); two rows'
+	// counts to a word.
+	uint32_t s01 = uint32_t(__popc(sig4 & 0xffu)) | (uint32_t(__popc(sig4 & 0xff00u)) << 16),
+	         s23 = uint32_t(__popc(sig4 & 0xff0000u)) | (uint32_t(__popc(sig4 & 0xff000000u)) << 16);
+	const uint32_t n01 = s01, n23 = s23;
+#pragma unroll
+	for (int o = 1; o < 32; o *= 2)
+	{
+		const uint32_t a = __shfl_up_sync(full, s01, o), b = __shfl_up_sync(full, s23, o);
+		if (lane >= o)
+		{
+			s01 += a;
+			s23 += b;
+		}
+	}
+	const uint32_t t01 = __shfl_sync(full, s01, 31), t23 = __shfl_sync(full, s23, 31);
+	s01 -= n01;
+	s23 -= n23;
+	const uint32_t total = (t01 & 0xffffu) + (t01 >> 16) + (t23 & 0xffffu) + (t23 >> 16);
+	const bool signs_staged = sign_bit + total <= 32 * rd.count;
+	const BlockReader<true> checked{rd.s, rd.off, rd.count, rd.g};
+#pragma unroll
+	for (int h = 0; h < 4; h++)
+	{
+		const uint32_t sig = (sig4 >> (8 * h)) & 0xffu;
+		if (((ballot >> (4 * h)) & 0xfu) != 0)
+		{
+			const uint32_t bit = sign_bit + (((h < 2 ? s01 : s23) >> (16 * (h & 1))) & 0xffffu);
+			uint32_t signs = 0;
+			if (sig != 0)
+				signs = signs_staged ? __funnelshift_r(rd.s[bit >> 5], rd.s[(bit >> 5) + 1], bit & 31u)
+				                     : __funnelshift_r(checked.w32(bit >> 5), checked.w32((bit >> 5) + 1), bit & 31u);
+#pragma unroll
+			for (int i = 0; i < 8; i++)
+			{
+				const bool on = (sig >> i) & 1u;
+				v[h][i] = on ? __uint_as_float(__float_as_uint(v[h][i]) ^ (signs << 31)) : 0.0f;
+				signs >>= on ? 1 : 0;
+			}
+			sign_bit += ((h < 2 ? t01 : t23) >> (16 * (h & 1))) & 0xffffu;
+		}
+		store_subblock(in.coef32, in.coef16, f16, at + int64_t(8 * h) * pitch, pitch, v[h]);
+	}
+}
+
+// One 32x32 block per warp, four 4x2 sub-blocks per lane (8x8 rows 0..3 of
+// column lane >> 3, sub-block lane & 7: the reference's mapping,
+// wavelet_dequant.comp:222-238). No CTA barrier: the block's words are staged in
+// the warp's shared memory, the header's prefixes are warp scans. Planes and
+// signs that lie inside the staged words (every valid block's) are read without
+// per-word checks; the area has room for the words just past them that a
+// window may touch. Bound by instruction issue at 4K, by latency at 1080p.
+// Measured against two sub-blocks per thread of a 64-thread CTA: decode of a 4K
+// 4:4:4 frame (1.2 MB) 118 -> 105 us, 1080p 32.8 -> 31.9 us.
+//
+// The warp with `clear_error` set clears the decode's error word: every
+// inverse level runs after the dequantiser has completed, so the clear precedes
+// any error report.
+__device__ __forceinline__ void dequant_body(DequantShared &sh, const BlockParams &p, const DecodeInput &in,
+                                             const int blk, const bool clear_error)
+{
+	const unsigned full = 0xffffffffu;
 	pdl_trigger();
-	const int k = find_band(p, blk);
-	const BandEntry &B = p.band[k];
+	const BandEntry &B = p.band[find_band(p, blk)];
 	const LevelDesc &L = p.level[B.level];
 	const int rel = blk - B.block32_offset;
 	const int by32 = rel / B.block32_stride, bx32 = rel - by32 * B.block32_stride;
 	const bool f16 = L.fp16 != 0;
-	const int t = threadIdx.x & (kGroup - 1), lane = t & 31;
-	const int sub = t & 7, lx = (t >> 3) & 3, ly0 = t >> 5;
-	const int ox = bx32 * 32 + lx * 8 + sub_x(sub);
+	const int lane = threadIdx.x & 31, sub = lane & 7, lx = lane >> 3;
+	const int pitch = L.pitch;
+	const int64_t at = B.offset + int64_t(by32 * 32 + sub_y(sub)) * pitch + bx32 * 32 + lx * 8 + sub_x(sub);
 	pdl_wait();
-	if (clear_error && t == 0 && in.error)
+	if (clear_error && lane == 0 && in.error)
 		*in.error = 0u;
-	if (clear_error && in.state && t < int(sizeof(DecodeState) / 4))
-		reinterpret_cast<uint32_t *>(in.state)[t] = 0u;
+	if (clear_error && in.state && lane < int(sizeof(DecodeState) / 4))
+		reinterpret_cast<uint32_t *>(in.state)[lane] = 0u;
 
 	uint32_t off, words = 0;
 	const bool sized_by_header = in.offsets || in.keys;
@@ -153,11 +274,8 @@ __device__ __forceinline__ void dequant_body(DequantShared &sh, const BlockParam
 		// Missing block: all coefficients are zero (wavelet_dequant.comp:242-248).
 		const float zero[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-		for (int h = 0; h < kSubs; h++)
-		{
-			const int oy = by32 * 32 + (ly0 + h * kRowStep) * 8 + sub_y(sub);
-			store_subblock(in.coef32, in.coef16, f16, B.offset + int64_t(oy) * L.pitch + ox, L.pitch, zero);
-		}
+		for (int h = 0; h < 4; h++)
+			store_subblock(in.coef32, in.coef16, f16, at + int64_t(8 * h) * pitch, pitch, zero);
 		return;
 	}
 
@@ -166,170 +284,51 @@ __device__ __forceinline__ void dequant_body(DequantShared &sh, const BlockParam
 	// table the size comes from the block header, so the first
 	// kSpeculativeWords are fetched together with it.
 	const PayloadReader grd{in.payload, in.payload_words};
+	uint32_t *const s = sh.words;
 	uint32_t staged;
 	if (sized_by_header)
 	{
-		stage_words<kGroup>(s_words, grd, off, 0, kSpeculativeWords, t);
-		block_sync<kSubs>(bar);
-		words = (s_words[0] >> 16) & 0xfffu;
+		stage_words(s, grd, off, 0, kSpeculativeWords);
+		__syncwarp();
+		words = (s[0] >> 16) & 0xfffu;
 		staged = min(max(words, kSpeculativeWords), uint32_t(kMaxBlockWords));
-		stage_words<kGroup>(s_words, grd, off, kSpeculativeWords, staged, t);
+		stage_words(s, grd, off, kSpeculativeWords, staged);
 	}
 	else
 	{
 		staged = min(words, uint32_t(kMaxBlockWords));
-		stage_words<kGroup>(s_words, grd, off, 0, staged, t);
+		stage_words(s, grd, off, 0, staged);
 	}
-	block_sync<kSubs>(bar);
-	const StagedReader rd{s_words, off, staged, grd};
-	const uint32_t ballot = rd.w32(off) & 0xffffu;
-	const uint32_t q_code = rd.w32(off + 1) & 0xffu;
+	__syncwarp();
+
+	// Header: lane t < 16 reads 8x8 t and finds where its planes start.
+	const BlockReader<true> checked{s, off, staged, grd};
+	const uint32_t ballot = checked.w32(0) & 0xffffu;
+	const float quant = decode_quant(checked.w32(1) & 0xffu);
 	const uint32_t n = uint32_t(__popc(ballot));
-
-	if (t < 16)
+	uint32_t header = 0; // code word, Q bits << 16, scale << 20
+	if (lane < 16 && ((ballot >> lane) & 1u))
 	{
-		uint32_t cw = 0, qb = 0;
-		if ((ballot >> t) & 1u)
-		{
-			const uint32_t local = uint32_t(__popc(ballot & ((1u << t) - 1u)));
-			cw = rd.u16(off * 2 + 4 + local);
-			qb = rd.u8(off * 4 + 8 + n * 2 + local) & 0xfu;
-		}
-		const uint32_t lsbs = cw & 0x5555u;
-		uint32_t msbs = cw & 0xaaaau;
-		msbs |= msbs >> 1;
-		const uint32_t cost = uint32_t(__popc(lsbs) + __popc(msbs)) + qb * 8u;
-		uint32_t inc = cost;
-#pragma unroll
-		for (int o = 1; o < 16; o *= 2)
-		{
-			const uint32_t y = __shfl_up_sync(0x0000ffffu, inc, o);
-			if (t >= o)
-				inc += y;
-		}
-		const uint32_t base = off * 4 + 8 + 3 * n;
-		s_plane_off[t] = base + inc - cost;
-		if (t == 15)
-			s_sign_base = 8u * (base + inc);
+		const uint32_t local = uint32_t(__popc(ballot & ((1u << lane) - 1u)));
+		header = checked.u16(4 + local) | (checked.u8(8 + n * 2 + local) << 16);
 	}
-	block_sync<kSubs>(bar);
-
-	float v[kSubs][8];
+	const uint32_t cost = uint32_t(plane_code_sum(header, 0)) + ((header >> 16) & 0xfu) * 8u;
+	uint32_t inc = cost;
 #pragma unroll
-	for (int h = 0; h < kSubs; h++)
+	for (int o = 1; o < 16; o *= 2)
 	{
-		const int grp = (ly0 + h * kRowStep) * 4 + lx;
-#pragma unroll
-		for (int i = 0; i < 8; i++)
-			v[h][i] = 0.0f;
-		if ((ballot >> grp) & 1u)
-		{
-			const uint32_t local = uint32_t(__popc(ballot & ((1u << grp) - 1u)));
-			const uint32_t cw = rd.u16(off * 2 + 4 + local);
-			const uint32_t cw2 = rd.u8(off * 4 + 8 + n * 2 + local);
-			const uint32_t qb = cw2 & 0xfu;
-			if (cw != 0)
-			{
-				const uint32_t mask = (1u << (2 * sub)) - 1u;
-				const uint32_t lsbs = cw & 0x5555u;
-				uint32_t msbs = cw & 0xaaaau;
-				msbs |= msbs >> 1;
-				uint32_t byte_offset =
-				    uint32_t(__popc(lsbs & mask) + __popc(msbs & mask)) + qb * uint32_t(sub) + s_plane_off[grp];
-				const int planes = int(qb + ((cw >> (2 * sub)) & 3u));
-				uint32_t dec[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-				if (planes <= 16)
-				{
-					// Plane bytes (most significant first) as the rows of two 8x8 bit
-					// matrices; transposed, byte i holds coefficient i's magnitude bits.
-					unsigned long long lo = 0, hi = 0;
-					for (int pl = planes - 1; pl >= 0; pl--)
-					{
-						const unsigned long long bits = rd.u8(byte_offset++);
-						if (pl < 8)
-							lo |= bits << (8 * pl);
-						else
-							hi |= bits << (8 * (pl - 8));
-					}
-					lo = transpose8x8(lo);
-					hi = transpose8x8(hi);
-#pragma unroll
-					for (int i = 0; i < 8; i++)
-						dec[i] = uint32_t((lo >> (8 * i)) & 0xffu) | (uint32_t((hi >> (8 * i)) & 0xffu) << 8);
-				}
-				else
-				{
-					// Only a malformed header gives more than 16 planes.
-					for (int pl = planes - 1; pl >= 0; pl--)
-					{
-						const uint32_t bits = rd.u8(byte_offset++);
-#pragma unroll
-						for (int i = 0; i < 8; i++)
-							dec[i] |= ((bits >> i) & 1u) << pl;
-					}
-				}
-#pragma unroll
-				for (int i = 0; i < 8; i++)
-				{
-					float f = float(dec[i]);
-					if (f != 0.0f)
-						f = __fadd_rn(f, 0.5f);
-					v[h][i] = f;
-				}
-			}
-			const float inv_scale = __fmul_rn(decode_quant(q_code), decode_quant_scale((cw2 >> 4) & 0xfu));
-#pragma unroll
-			for (int i = 0; i < 8; i++)
-				v[h][i] = __fmul_rn(v[h][i], inv_scale);
-		}
+		const uint32_t y = __shfl_up_sync(full, inc, o);
+		if (lane >= o)
+			inc += y;
 	}
-
-	// Sign bits: position = number of significant coefficients before this one
-	// (in sub-block order: 8x8 rows, then the 32 sub-blocks of a row).
-	uint32_t nsig[kSubs], inc[kSubs];
-#pragma unroll
-	for (int h = 0; h < kSubs; h++)
-	{
-		nsig[h] = 0;
-#pragma unroll
-		for (int i = 0; i < 8; i++)
-			nsig[h] += v[h][i] != 0.0f ? 1u : 0u;
-		inc[h] = nsig[h];
-#pragma unroll
-		for (int o = 1; o < 32; o *= 2)
-		{
-			const uint32_t y = __shfl_up_sync(0xffffffffu, inc[h], o);
-			if (lane >= o)
-				inc[h] += y;
-		}
-		if (lane == 31)
-			s_sig[ly0 + h * kRowStep] = inc[h];
-	}
-	block_sync<kSubs>(bar);
-#pragma unroll
-	for (int h = 0; h < kSubs; h++)
-	{
-		const int ly = ly0 + h * kRowStep;
-		uint32_t bitpos = s_sign_base + inc[h] - nsig[h];
-		for (int w = 0; w < ly; w++)
-			bitpos += s_sig[w];
-		// This thread's (at most 8) sign bits are consecutive: one 64-bit window.
-		const uint32_t sw = bitpos >> 5, shift = bitpos & 31u;
-		const uint64_t window = (uint64_t(rd.w32(sw + 1)) << 32 | rd.w32(sw)) >> shift;
-		int nth = 0;
-#pragma unroll
-		for (int i = 0; i < 8; i++)
-		{
-			if (v[h][i] != 0.0f)
-			{
-				if ((window >> nth) & 1u)
-					v[h][i] = -v[h][i];
-				nth++;
-			}
-		}
-		const int oy = by32 * 32 + ly * 8 + sub_y(sub);
-		store_subblock(in.coef32, in.coef16, f16, B.offset + int64_t(oy) * L.pitch + ox, L.pitch, v[h]);
-	}
+	const uint32_t base = 8 + 3 * n;
+	const uint32_t plane_end = base + __shfl_sync(full, inc, 15);
+	const uint32_t first_byte = base + inc - cost;
+	if (plane_end <= 4 * staged)
+		dequant_block(BlockReader<false>{s, off, staged, grd}, ballot, header, first_byte, 8u * plane_end, quant, in, f16, at,
+		              pitch);
+	else
+		dequant_block(checked, ballot, header, first_byte, 8u * plane_end, quant, in, f16, at, pitch);
 }
 
 constexpr int kBandTile = 36; // 32 band samples + 2 on each side

@@ -344,11 +344,6 @@ __device__ __forceinline__ void store_subblock(float *c32, __half *c16, bool fp1
 	}
 }
 
-// Barrier of one 128-thread group of a CTA (hardware barrier `id`, 1 or 2):
-// the block-level bodies (packing, dequantisation) run one 32x32 block per
-// group, so a CTA of 256 threads can hold two independent blocks.
-__device__ __forceinline__ void group_sync(int id) { asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory"); }
-
 // Cooperative copy of a parameter struct from global to shared memory (the
 // caller synchronises before use).
 template <typename T> __device__ __forceinline__ void load_params(T &dst, const T &src)
@@ -430,44 +425,30 @@ __device__ __forceinline__ void compute_quant_scale(float max_wave, uint32_t &co
 	}
 }
 
-// Required plane bytes of an 8x8 block (block_packing.comp:97-105).
-__device__ __forceinline__ uint32_t required_8x8_bytes(uint32_t cw)
+// Sum over the eight plane codes p of cw of max(p - d, 0), d = 0, 1 or 2.
+__device__ __forceinline__ int plane_code_sum(uint32_t cw, int d)
 {
-	uint32_t q_bits = (cw >> kQPlanesOffset) & 0xfu;
-	uint32_t lsbs = cw & 0x5555u;
-	uint32_t msbs = cw & 0xaaaau;
-	msbs |= msbs >> 1;
-	return uint32_t(__popc(lsbs) + __popc(msbs)) + q_bits * 8u;
+	const uint32_t l = cw & 0x5555u, m = (cw >> 1) & 0x5555u, lm = l & m;
+	const uint32_t bits = d <= 0 ? (l | ((m | (m << 1)) << 16)) : (d == 1 ? (m | (lm << 1)) : lm);
+	return __popc(bits);
 }
 
 // Drop `quant` planes from a code word (block_packing.comp:107-142): first the
 // Q planes, then max(code - rest, 0) per 4x2 sub-block.
 __device__ __forceinline__ uint32_t quantize_code_word(uint32_t cw, int quant)
 {
-	if (quant != 0 && cw != 0)
-	{
-		int q_bits = int((cw >> kQPlanesOffset) & 0xfu);
-		int sub = min(q_bits, quant);
-		q_bits -= sub;
-		quant -= sub;
-		if (quant != 0)
-		{
-			quant = min(quant, 3);
-			uint32_t p0 = cw & 0x5555u;
-			uint32_t p1 = (cw & 0xaaaau) >> 1;
-			uint32_t p2 = p0 & p1;
-			for (int i = 0; i < quant; i++)
-			{
-				p0 = p1;
-				p1 = p2;
-				p2 = 0;
-			}
-			p0 &= ~p1;
-			cw = (cw & ~0xffffu) | ((p0 | (p1 << 1)) & 0xffffu);
-		}
-		cw = (cw & ~(0xfu << kQPlanesOffset)) | (uint32_t(q_bits) << kQPlanesOffset);
-	}
-	return cw;
+	const int q_bits = int((cw >> kQPlanesOffset) & 0xfu);
+	const int rest = quant - q_bits;
+	const uint32_t l = cw & 0x5555u, m = (cw >> 1) & 0x5555u;
+	// Codes 3, 2, 1 become 2, 1, 0 with one plane dropped and 1, 0, 0 with two.
+	uint32_t codes = cw & 0xffffu;
+	if (rest == 1)
+		codes = (m & ~l) | ((m & l) << 1);
+	else if (rest == 2)
+		codes = m & l;
+	else if (rest > 2)
+		codes = 0;
+	return (cw & ~((0xfu << kQPlanesOffset) | 0xffffu)) | codes | (uint32_t(max(-rest, 0)) << kQPlanesOffset);
 }
 
 // block_packing.comp:161-167

@@ -1393,7 +1393,7 @@ struct pyrowave_decoder_opaque
 				cudaMemsetAsync(state_d, 0, sizeof(DecodeState), s);
 			if (dequant)
 			{
-				launch_dequant(bp, in, 0, g.block_count_32x32, false, s);
+				launch_dequant(bp, in, false, s);
 				ok = ok && last_captured_node(s, node_dequant);
 				timing.mark(device, s, "dequant");
 			}
@@ -1420,8 +1420,7 @@ struct pyrowave_decoder_opaque
 			bool ok = true;
 			if (dequant)
 			{
-				int first = 0;
-				ok = set_kernel_args(graph.exec, node_dequant, bp, din, first);
+				ok = set_kernel_args(graph.exec, node_dequant, bp, din);
 			}
 			for (int level = 0; level < kLevels; level++)
 				ok = ok && set_kernel_args(graph.exec, dequant ? node_idwt_full[level] : node_idwt_only[level], lp[level],
@@ -2832,8 +2831,8 @@ struct pyrowave_cuda_batch_opaque
 		}
 		n[kStageQuant] = (fr.small_blocks + 1) / 2;
 		n[kStageResolve] = fr.slices;
-		n[kStagePack] = (fr.block_count + 1) / 2;
-		n[kStageDequant] = (fr.block_count + 1) / 2;
+		n[kStagePack] = (fr.block_count + kBatchBlockItem - 1) / kBatchBlockItem;
+		n[kStageDequant] = n[kStagePack];
 	}
 
 	// Work lists and gates of the persistent mode: stage by stage, every frame's

@@ -369,8 +369,9 @@ constexpr int kMaxBatchFrames = 256;
 constexpr int kStageDwt0 = 0;     // forward level L is stage kStageDwt0 + L (levels 0..4)
 constexpr int kStageQuant = 5;    // quantiser of the transform-only levels, two 32x32 blocks per item
 constexpr int kStageResolve = 6;  // rate-control slices
-constexpr int kStagePack = 7;     // two 32x32 blocks per item
-constexpr int kStageDequant = 8;  // two 32x32 blocks per item
+constexpr int kStagePack = 7;     // kBatchBlockItem 32x32 blocks per item
+constexpr int kStageDequant = 8;  // kBatchBlockItem 32x32 blocks per item
+constexpr int kBatchBlockItem = 8;
 constexpr int kStageIdwt4 = 9;    // inverse level L is stage kStageIdwt4 + 4 - L
 constexpr int kBatchStages = 14;
 constexpr int kBatchLocalBits = 19;
@@ -428,9 +429,8 @@ void launch_quant_pretransformed(const BlockParams &p, const EncodeBuffers &buf,
 int resolve_cluster_max();
 void launch_resolve(const ResolveParams &p, const EncodeBuffers &buf, cudaStream_t stream);
 void launch_pack(const BlockParams &p, const EncodeBuffers &buf, cudaStream_t stream);
-// Dequantise blocks [first, first + count) (block index order).
-void launch_dequant(const BlockParams &p, const DecodeInput &in, int first, int count, bool programmatic,
-                    cudaStream_t stream);
+// Dequantise every block of the frame.
+void launch_dequant(const BlockParams &p, const DecodeInput &in, bool programmatic, cudaStream_t stream);
 void launch_idwt_level(const LevelParams &p, const DecodeInput &in, const PlaneOutput &out, const LevelTileMap *maps,
                        bool programmatic,
                        cudaStream_t stream);
