@@ -37,18 +37,12 @@ __global__ void __launch_bounds__(32) dequant_batch_kernel(const BatchFrame *fra
 	dequant_body(sh, s_p, s_in, local, local == 0);
 }
 
-// 256-thread CTAs: three per SM (80 registers) for levels of about one wave,
-// four per SM (64 registers) for levels of several waves, each measured the
-// faster of the two there; 1024-thread CTAs keep 32 registers.
-template <int kThreads> constexpr int kIdwtMinBlocks = kThreads >= 1024 ? 2 : 3;
-constexpr int kIdwtManyTiles = 2 * 148 * 4; // levels with at least this many tiles use four CTAs per SM
-
-template <int kThreads, int kMinBlocks = kIdwtMinBlocks<kThreads>>
-__global__ void __launch_bounds__(kThreads, kMinBlocks) idwt_kernel(const LevelParams p, const DecodeInput in, const PlaneOutput out,
-                                                                     const __grid_constant__ LevelTileMap maps)
+template <bool kHalf>
+__global__ void __launch_bounds__(256, 4) idwt_kernel(const LevelParams p, const DecodeInput in, const PlaneOutput out,
+                                                      const __grid_constant__ LevelTileMap maps)
 {
 	__shared__ IdwtShared sh;
-	idwt_body<kThreads>(sh, p, in, out, &maps, int(blockIdx.x), int(blockIdx.y));
+	idwt_body<256, 1, kHalf>(sh, p, in, out, &maps, int(blockIdx.x), int(blockIdx.y));
 }
 
 // Small levels (fewer tiles than SMs): four 256-thread CTAs per tile, one per
@@ -56,18 +50,19 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) idwt_kernel(const LevelP
 constexpr int kIdwtStripes = 4;
 // Same parameters as idwt_kernel (graph nodes are updated with one argument
 // list); the stripes load with plain vector loads, not tensor maps.
+template <bool kHalf>
 __global__ void __launch_bounds__(256, 4) idwt_stripes_kernel(const LevelParams p, const DecodeInput in, const PlaneOutput out,
                                                               const __grid_constant__ LevelTileMap maps)
 {
 	(void)maps;
 	__shared__ IdwtSharedT<IdwtSplit<256, kIdwtStripes>::kOutRows> sh;
-	idwt_body<256, kIdwtStripes>(sh, p, in, out, nullptr, int(blockIdx.x) / kIdwtStripes, int(blockIdx.y),
-	                             int(blockIdx.x) % kIdwtStripes);
+	idwt_body<256, kIdwtStripes, kHalf>(sh, p, in, out, nullptr, int(blockIdx.x) / kIdwtStripes, int(blockIdx.y),
+	                                    int(blockIdx.x) % kIdwtStripes);
 }
 
-// Batched form: one CTA per (frame, component, tile) of this level.
-template <int kThreads, int kMinBlocks = kIdwtMinBlocks<kThreads>>
-__global__ void __launch_bounds__(kThreads, kMinBlocks) idwt_batch_kernel(const BatchFrame *frames, const BatchFrameIO *io,
+// Batched form (FP32 storage): one CTA per (frame, component, tile) of this level.
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads, kThreads >= 1024 ? 2 : 4) idwt_batch_kernel(const BatchFrame *frames, const BatchFrameIO *io,
                                                               const uint32_t *cta_map, const int level,
                                                               const __grid_constant__ BatchTileMaps maps)
 {
@@ -82,8 +77,8 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) idwt_batch_kernel(const 
 	__syncthreads();
 	const int ntiles = s_p.L.tiles_x * s_p.L.tiles_y;
 	__shared__ IdwtShared sh;
-	idwt_body<kThreads>(sh, s_p, s_in, s_out, f < kBatchTileMapFrames ? &maps.frame[f] : nullptr, local % ntiles,
-	                    local / ntiles);
+	idwt_body<kThreads, 1, false>(sh, s_p, s_in, s_out, f < kBatchTileMapFrames ? &maps.frame[f] : nullptr,
+	                              local % ntiles, local / ntiles);
 }
 
 // Canonical pyramid (all transmitted bands, band-major, unpadded) <-> padded storage.
@@ -122,27 +117,6 @@ void launch_dequant(const BlockParams &p, const DecodeInput &in, bool programmat
 	cudaLaunchKernelEx(&lc.cfg, dequant_kernel, p, in);
 }
 
-// SMs of the current device (queried once).
-int device_sm_count()
-{
-	static int cached = 0;
-	if (cached == 0)
-	{
-		int dev = 0, n = 0;
-		if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-		    n <= 0)
-		{
-			(void)cudaGetLastError();
-			n = 148;
-		}
-		cached = n;
-	}
-	return cached;
-}
-
-// Levels that fit one wave at three CTAs per SM run the 80-register CTAs (the
-// faster per tile); larger levels run four 64-register CTAs per SM, so a level
-// just above one wave at three (1080p level 0: 510 tiles) still runs in one.
 void launch_idwt_level(const LevelParams &p, const DecodeInput &in, const PlaneOutput &out, const LevelTileMap *maps,
                        bool programmatic, cudaStream_t stream)
 {
@@ -150,20 +124,16 @@ void launch_idwt_level(const LevelParams &p, const DecodeInput &in, const PlaneO
 	LevelTileMap m = {};
 	if (maps)
 		m = *maps;
+	const bool half = p.L.fp16 || p.L.stage16 || (p.level > 0 && p.P.fp16);
 	if (int(grid.x * grid.y) < kSmallLevelTiles)
 	{
 		LaunchConfig lc(dim3(grid.x * kIdwtStripes, grid.y), dim3(256), stream, programmatic);
-		cudaLaunchKernelEx(&lc.cfg, idwt_stripes_kernel, p, in, out, m);
-	}
-	else if (int(grid.x * grid.y) <= 3 * device_sm_count())
-	{
-		LaunchConfig lc(grid, dim3(256), stream, programmatic);
-		cudaLaunchKernelEx(&lc.cfg, idwt_kernel<256>, p, in, out, m);
+		cudaLaunchKernelEx(&lc.cfg, half ? idwt_stripes_kernel<true> : idwt_stripes_kernel<false>, p, in, out, m);
 	}
 	else
 	{
 		LaunchConfig lc(grid, dim3(256), stream, programmatic);
-		cudaLaunchKernelEx(&lc.cfg, idwt_kernel<256, 4>, p, in, out, m);
+		cudaLaunchKernelEx(&lc.cfg, half ? idwt_kernel<true> : idwt_kernel<false>, p, in, out, m);
 	}
 }
 
@@ -190,15 +160,10 @@ void launch_idwt_batch(const BatchFrame *frames, const BatchFrameIO *io, const u
 		LaunchConfig lc(dim3(nctas), dim3(1024), stream, programmatic);
 		cudaLaunchKernelEx(&lc.cfg, idwt_batch_kernel<1024>, frames, io, cta_map, level, m);
 	}
-	else if (nctas < kIdwtManyTiles)
-	{
-		LaunchConfig lc(dim3(nctas), dim3(256), stream, programmatic);
-		cudaLaunchKernelEx(&lc.cfg, idwt_batch_kernel<256>, frames, io, cta_map, level, m);
-	}
 	else
 	{
 		LaunchConfig lc(dim3(nctas), dim3(256), stream, programmatic);
-		cudaLaunchKernelEx(&lc.cfg, idwt_batch_kernel<256, 4>, frames, io, cta_map, level, m);
+		cudaLaunchKernelEx(&lc.cfg, idwt_batch_kernel<256>, frames, io, cta_map, level, m);
 	}
 }
 

@@ -462,7 +462,10 @@ __device__ __forceinline__ void quantise_samples2(f32x2 e, float scale, uint32_t
 // lifting: decode of a 1080p 4:2:0 frame 41.7 -> 32.8 us, 4K 4:4:4 133 -> 118 us;
 // 16-bit 4:4:4 at 1365x767 (rows of no common alignment) encode + decode 124 ->
 // 96 us.
-template <int kThreads, int kStripes = 1>
+//
+// kHalf: the level, or the finer one it writes, is stored in FP16, or lifting is
+// staged through it; the all-FP32 form carries none of that code.
+template <int kThreads, int kStripes, bool kHalf>
 __device__ __forceinline__ void idwt_body(IdwtSharedT<IdwtSplit<kThreads, kStripes>::kOutRows> &sh, const LevelParams &p,
                                           const DecodeInput &in, const PlaneOutput &out, const LevelTileMap *maps,
                                           const int tile, const int comp_index, const int stripe = 0)
@@ -477,7 +480,7 @@ __device__ __forceinline__ void idwt_body(IdwtSharedT<IdwtSplit<kThreads, kStrip
 	const int tx = tile % L.tiles_x, ty = tile / L.tiles_x;
 	const int nx = L.width, ny = L.height;
 	const bool final_level = level == 0 || (level == 1 && comp != 0 && !p.chroma444);
-	const bool f16 = L.fp16 != 0;
+	const bool f16 = kHalf && L.fp16 != 0, stage16 = kHalf && L.stage16 != 0;
 
 	// Interior tiles read every band sample at its own position. Interior FP32
 	// tiles of a decoder with tensor maps take one TMA box per band (barrier and
@@ -488,7 +491,7 @@ __device__ __forceinline__ void idwt_body(IdwtSharedT<IdwtSplit<kThreads, kStrip
 	const bool y_inside = y0 >= 0 && y0 + kRows <= ny;
 	const bool interior = x0 >= 0 && x0 + kBandRow <= nx && y_inside;
 	const bool use_tma = kThreads == 256 && kStripes == 1 && interior && maps && ((maps->valid >> comp) & 1u) && !f16 &&
-	                     !L.stage16;
+	                     !stage16;
 	if (!interior)
 	{
 		for (int k = threadIdx.x; k < 2 * kBandRow + 2 * kRows; k += kThreads)
@@ -589,7 +592,7 @@ __device__ __forceinline__ void idwt_body(IdwtSharedT<IdwtSplit<kThreads, kStrip
 				continue;
 			const int b = br / kRows, i = br - b * kRows;
 			float4 f = v[u];
-			if (L.stage16)
+			if (stage16)
 			{
 				f.x = round_to_half(f.x);
 				f.y = round_to_half(f.y);
@@ -627,7 +630,7 @@ __device__ __forceinline__ void idwt_body(IdwtSharedT<IdwtSplit<kThreads, kStrip
 #pragma unroll
 			for (int jj = 4; jj < 4 + kOut; jj++)
 			{
-				if (L.stage16)
+				if (stage16)
 				{
 					float a, b;
 					f2_unpack(e[jj], a, b);
@@ -675,7 +678,7 @@ __device__ __forceinline__ void idwt_body(IdwtSharedT<IdwtSplit<kThreads, kStrip
 			}
 		}
 		lift_inverse2(e);
-		if (L.stage16)
+		if (stage16)
 		{
 #pragma unroll
 			for (int jj = 4; jj < 4 + kOut; jj++)
@@ -733,7 +736,7 @@ __device__ __forceinline__ void idwt_body(IdwtSharedT<IdwtSplit<kThreads, kStrip
 		{
 			const LevelDesc &P = p.P;
 			const int64_t ll = comp == 0 ? p.prev_ll[0] : (comp == 1 ? p.prev_ll[1] : p.prev_ll[2]);
-			const bool pf16 = P.fp16 != 0;
+			const bool pf16 = kHalf && P.fp16 != 0;
 			float r[2][kOut];
 #pragma unroll
 			for (int k = 0; k < kOut; k++)

@@ -406,8 +406,10 @@ __device__ __forceinline__ float decode_quant(uint32_t code)
 
 __device__ __forceinline__ int find_msb(uint32_t v) { return v ? 31 - __clz(v) : -1; }
 
-// 8-bit quant scale per 8x8 block (wavelet_quant.comp:95-111).
-__device__ __forceinline__ void compute_quant_scale(float max_wave, uint32_t &code, float &scale)
+// 8-bit quant scale per 8x8 block (wavelet_quant.comp:95-111): with target =
+// 2^e - 0.25 from the maximum's exponent, code = ceil((max / target - 0.25) * 8),
+// scale = 1 / (code / 8 + 0.25).
+__device__ __forceinline__ void compute_quant_scale_any(float max_wave, uint32_t &code, float &scale)
 {
 	if (max_wave < 1.0f)
 	{
@@ -423,6 +425,30 @@ __device__ __forceinline__ void compute_quant_scale(float max_wave, uint32_t &co
 		code = uint32_t(ceilf(__fmul_rn(__fsub_rn(inv_scale, 0.25f), 8.0f)));
 		scale = __fdiv_rn(1.0f, decode_quant_scale(code));
 	}
+}
+
+// The same without a division, for maxima below kQuantScaleFast (every 8-bit or
+// 16-bit frame's). (code + 2) / 8 is a float, and no float m has m / target
+// above it by half a unit in its last place or less: target < 2^e makes the step
+// from target * (code + 2) / 8, exact in 24 bits, to the next float larger than
+// that. So the rounded quotient compares with (code + 2) / 8 as the exact one
+// does, and code + 2 = k is the smallest integer with 8 max <= target * k: an
+// estimate that is k or k - 1, then one exact comparison. A maximum below 1 has
+// k = 8.
+constexpr float kQuantScaleFast = 262144.0f;
+__device__ __forceinline__ void compute_quant_scale(float max_wave, uint32_t &code, float &scale)
+{
+	const int e = int(__float_as_uint(__fsub_rn(max_wave, 0.25f)) >> 23) - 126;
+	const float target4 = __fsub_rn(__int_as_float((e + 129) << 23), 1.0f), max32 = __fmul_rn(max_wave, 32.0f);
+	float r;
+	asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(target4));
+	float k = ceilf(__fmul_rn(__fmul_rn(max32, r), 1.0f - 0x1p-21f));
+	if (max32 > __fmul_rn(target4, k))
+		k = __fadd_rn(k, 1.0f);
+	if (max_wave < 1.0f)
+		k = 8.0f;
+	code = uint32_t(int(k)) - 2u;
+	scale = __frcp_rn(__fmul_rn(k, 0.125f));
 }
 
 // Sum over the eight plane codes p of cw of max(p - d, 0), d = 0, 1 or 2.

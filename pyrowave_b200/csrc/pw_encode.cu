@@ -106,7 +106,10 @@ __device__ __forceinline__ void quant_analyze_row(const float *tile, const int l
 
 	uint32_t qcode;
 	float qs;
-	compute_quant_scale(max_wave, qcode, qs);
+	if (__any_sync(full, max_wave >= kQuantScaleFast))
+		compute_quant_scale_any(max_wave, qcode, qs);
+	else
+		compute_quant_scale(max_wave, qcode, qs);
 	float av[8];
 #pragma unroll
 	for (int i = 0; i < 8; i++)
@@ -156,7 +159,7 @@ __device__ __forceinline__ void quant_analyze_row(const float *tile, const int l
 	}
 
 	const float overall = __fmul_rn(qres, qs);
-	const float inv_quant = __fdiv_rn(1.0f, overall);
+	const float inv_quant = __frcp_rn(overall);
 	const float iqs = __fmul_rn(inv_quant, inv_quant);
 	const float rdo = B.rdo_scale;
 
@@ -396,9 +399,10 @@ constexpr int kLargeLevelThreads = 256;
 // the subtraction are: the quotient is u * hi + (u * lo rounded), with 1 / n =
 // hi + lo, fused, which equals the rounded quotient for every u in [0, n]
 // (checked for all of them). Two samples at a time; bits holds 2^23 + u.
-__device__ __forceinline__ f32x2 unorm_centered2(uint32_t bits0, uint32_t bits1, bool sample16)
+template <int kMax> __device__ __forceinline__ f32x2 unorm_centered2(uint32_t bits0, uint32_t bits1)
 {
-	const float hi = sample16 ? 0x1.0001p-16f : 0x1.010102p-8f, lo = sample16 ? 0x1.0001p-48f : -0x1.fdfdfep-33f;
+	static_assert(kMax == 255 || kMax == 65535, "8-bit or 16-bit samples");
+	const float hi = kMax == 65535 ? 0x1.0001p-16f : 0x1.010102p-8f, lo = kMax == 65535 ? 0x1.0001p-48f : -0x1.fdfdfep-33f;
 	const f32x2 u = f2_add_rn(f2_pack(__uint_as_float(bits0), __uint_as_float(bits1)), f2_pack(-8388608.0f, -8388608.0f));
 	const f32x2 q = f2_fma_rn(u, f2_pack(hi, hi), f2_mul_rn(u, f2_pack(lo, lo)));
 	return f2_add_rn(q, f2_pack(-0.5f, -0.5f));
@@ -535,7 +539,10 @@ __device__ __forceinline__ void quant_tile(DwtShared &sh, const LevelParams &p, 
 // Measured against scalar lifting with TMA loads and a table of converted
 // samples: encode of a 720p 4:2:0 frame 37.9 -> 34.9 us, 1080p 49.2 -> 47.5 us,
 // 4K 4:4:4 (1.2 MB) 183 -> 179 us.
-template <int kThreads, int kStripes = 1>
+//
+// kHalf: the level or its input is stored in FP16 or staged through it; the
+// all-FP32 form carries none of that code.
+template <int kThreads, int kStripes, bool kHalf>
 __device__ __forceinline__ void dwt_forward_body(DwtSharedT<DwtSplit<kThreads, kStripes>::kRowsIn> &sh,
                                                  const LevelParams &p, const PlaneInput &in, const EncodeBuffers &buf,
                                                  const int fused, const int tile, const int comp_index,
@@ -592,105 +599,125 @@ __device__ __forceinline__ void dwt_forward_body(DwtSharedT<DwtSplit<kThreads, k
 		pdl_wait();
 
 	// Tile load: a thread takes rows r and r + kPairRows of its four columns,
-	// every load of its iterations in flight at once.
+	// every load of its iterations in flight at once. The few threads beyond
+	// the last full row of vectors, and rows beyond the window, repeat others'
+	// loads instead of branching.
 	constexpr int kLoadRows = kThreads / kVecs; // row pairs per iteration
 	constexpr int kIters = (kPairRows + kLoadRows - 1) / kLoadRows;
 	{
-		const int j = threadIdx.x % kVecs, pr0 = threadIdx.x / kVecs;
-		const bool loader = threadIdx.x < kLoadRows * kVecs;
+		const int j = threadIdx.x % kVecs, pr0 = min(int(threadIdx.x) / kVecs, kPairRows - 1);
 		// This thread's four columns are consecutive inside the source, or (edge) gathered.
-		const bool inside = x0 + 4 * j >= 0 && x0 + 4 * j + 4 <= res_w;
-		int4 xi = make_int4(x0 + 4 * j, x0 + 4 * j + 1, x0 + 4 * j + 2, x0 + 4 * j + 3);
-		if (!inside)
-			xi = *reinterpret_cast<const int4 *>(&sh.xidx[4 * j]);
+		const int x = x0 + 4 * j;
+		const bool inside = x >= 0 && x + 4 <= res_w;
+		auto pair_row = [&](int u) {
+			const int pr = pr0 + u * kLoadRows;
+			return (u + 1) * kLoadRows <= kPairRows ? pr : min(pr, kPairRows - 1);
+		};
 		auto row_of = [&](int i) { return y_inside ? y0 + i : sh.yidx[i]; };
-		auto put = [&](int pr, const f32x2 (&v)[4]) {
-			float *dst = &sh.in[pr][4 * j];
+		auto put = [&](int u, const f32x2 (&v)[4]) {
+			float *dst = &sh.in[pair_row(u)][4 * j];
 			*reinterpret_cast<ulonglong2 *>(dst) = make_ulonglong2(v[0], v[1]);
 			*reinterpret_cast<ulonglong2 *>(dst + kInOdd) = make_ulonglong2(v[2], v[3]);
+		};
+		auto half_stage = [&](f32x2 &v) {
+			if (kHalf && L.stage16)
+			{
+				float lo, hi;
+				f2_unpack(v, lo, hi);
+				v = f2_pack(round_to_half(lo), round_to_half(hi));
+			}
 		};
 		if (from_plane)
 		{
 			const uint8_t *src = comp == 0 ? in.data[0] : (comp == 1 ? in.data[1] : in.data[2]);
 			const int pitch = comp == 0 ? in.pitch[0] : (comp == 1 ? in.pitch[1] : in.pitch[2]);
 			const int xs = comp == 0 ? in.xstride[0] : (comp == 1 ? in.xstride[1] : in.xstride[2]);
-			const bool wide = in.sample16 != 0;
 			const uintptr_t align = reinterpret_cast<uintptr_t>(src) | uintptr_t(pitch);
-			uint2 raw[kIters][2];
-			if (!wide)
+			if (in.sample16)
 			{
-				const bool vec = inside && xs == 1 && (align & 3u) == 0;
-				// Unaligned rows: two aligned words around the four bytes, where the
-				// row has bytes on both sides of them.
-				const bool vec_shift = !vec && inside && xs == 1 && x0 + 4 * j >= 4 && x0 + 4 * j + 8 <= res_w;
+				uint2 raw[kIters][2];
+				const bool vec = inside && xs == 2 && (align & 7u) == 0;
+				int4 xi = make_int4(x, x + 1, x + 2, x + 3);
+				if (!inside)
+					xi = *reinterpret_cast<const int4 *>(&sh.xidx[4 * j]);
 #pragma unroll
 				for (int u = 0; u < kIters; u++)
 #pragma unroll
 					for (int h = 0; h < 2; h++)
 					{
-						const int pr = pr0 + u * kLoadRows;
-						raw[u][h].y = 0;
-						if (!loader || pr >= kPairRows)
-							raw[u][h].x = 0;
-						else
-						{
-							const uint8_t *row = src + size_t(row_of(pr + h * kPairRows)) * pitch;
-							if (vec)
-								raw[u][h].x = __ldg(reinterpret_cast<const uint32_t *>(row + xi.x));
-							else if (vec_shift)
-							{
-								const uintptr_t a = reinterpret_cast<uintptr_t>(row + xi.x);
-								const uint32_t *w = reinterpret_cast<const uint32_t *>(a & ~uintptr_t(3));
-								raw[u][h].x = __funnelshift_r(__ldg(w), __ldg(w + 1), 8u * uint32_t(a & 3u));
-							}
-							else
-								raw[u][h].x = pack4_u8(row, xi, xs);
-						}
+						const uint8_t *row = src + size_t(row_of(pair_row(u) + h * kPairRows)) * pitch;
+						raw[u][h] = vec ? __ldg(reinterpret_cast<const uint2 *>(row + 2 * x)) : pack4_u16(row, xi, xs);
 					}
+#pragma unroll
+				for (int u = 0; u < kIters; u++)
+				{
+					f32x2 v[4];
+#pragma unroll
+					for (int b = 0; b < 4; b++)
+					{
+						uint32_t bits[2]; // sample b of a row over the exponent of 2^23
+#pragma unroll
+						for (int h = 0; h < 2; h++)
+							bits[h] = __byte_perm(b < 2 ? raw[u][h].x : raw[u][h].y, 0x4B000000u, (b & 1) ? 0x7432 : 0x7410);
+						v[b] = unorm_centered2<65535>(bits[0], bits[1]);
+						half_stage(v[b]);
+					}
+					put(u, v);
+				}
 			}
 			else
 			{
-				const bool vec = inside && xs == 2 && (align & 7u) == 0;
+				uint32_t raw[kIters][2];
+				if (x_inside && y_inside && xs == 1 && (align & 3u) == 0)
+				{
+					const uint8_t *at = src + size_t(y0 + pr0) * pitch + x;
+#pragma unroll
+					for (int u = 0; u < kIters; u++)
+#pragma unroll
+						for (int h = 0; h < 2; h++)
+							raw[u][h] = __ldg(reinterpret_cast<const uint32_t *>(
+							    at + size_t(uint32_t(pair_row(u) - pr0 + h * kPairRows)) * pitch));
+				}
+				else
+				{
+					const bool vec = inside && xs == 1 && (align & 3u) == 0;
+					// Unaligned rows: two aligned words around the four bytes, where the
+					// row has bytes on both sides of them.
+					const bool vec_shift = !vec && inside && xs == 1 && x >= 4 && x + 8 <= res_w;
+					int4 xi = make_int4(x, x + 1, x + 2, x + 3);
+					if (!inside)
+						xi = *reinterpret_cast<const int4 *>(&sh.xidx[4 * j]);
+#pragma unroll
+					for (int u = 0; u < kIters; u++)
+#pragma unroll
+						for (int h = 0; h < 2; h++)
+						{
+							const uint8_t *row = src + size_t(row_of(pair_row(u) + h * kPairRows)) * pitch;
+							if (vec)
+								raw[u][h] = __ldg(reinterpret_cast<const uint32_t *>(row + x));
+							else if (vec_shift)
+							{
+								const uintptr_t a = reinterpret_cast<uintptr_t>(row + x);
+								const uint32_t *w = reinterpret_cast<const uint32_t *>(a & ~uintptr_t(3));
+								raw[u][h] = __funnelshift_r(__ldg(w), __ldg(w + 1), 8u * uint32_t(a & 3u));
+							}
+							else
+								raw[u][h] = pack4_u8(row, xi, xs);
+						}
+				}
 #pragma unroll
 				for (int u = 0; u < kIters; u++)
-#pragma unroll
-					for (int h = 0; h < 2; h++)
-					{
-						const int pr = pr0 + u * kLoadRows;
-						if (!loader || pr >= kPairRows)
-							raw[u][h] = make_uint2(0, 0);
-						else
-						{
-							const uint8_t *row = src + size_t(row_of(pr + h * kPairRows)) * pitch;
-							raw[u][h] = vec ? __ldg(reinterpret_cast<const uint2 *>(row + 2 * xi.x)) : pack4_u16(row, xi, xs);
-						}
-					}
-			}
-#pragma unroll
-			for (int u = 0; u < kIters; u++)
-			{
-				const int pr = pr0 + u * kLoadRows;
-				if (!loader || pr >= kPairRows)
-					continue;
-				f32x2 v[4];
-#pragma unroll
-				for (int b = 0; b < 4; b++)
 				{
-					// Sample b of a row over the exponent of 2^23.
-					uint32_t bits[2];
+					f32x2 v[4];
 #pragma unroll
-					for (int h = 0; h < 2; h++)
-						bits[h] = wide ? __byte_perm(b < 2 ? raw[u][h].x : raw[u][h].y, 0x4B000000u, (b & 1) ? 0x7432 : 0x7410)
-						               : __byte_perm(raw[u][h].x, 0x4B000000u, 0x7440 + b);
-					v[b] = unorm_centered2(bits[0], bits[1], wide);
-					if (L.stage16)
+					for (int b = 0; b < 4; b++)
 					{
-						float lo, hi;
-						f2_unpack(v[b], lo, hi);
-						v[b] = f2_pack(round_to_half(lo), round_to_half(hi));
+						v[b] = unorm_centered2<255>(__byte_perm(raw[u][0], 0x4B000000u, 0x7440 + b),
+						                            __byte_perm(raw[u][1], 0x4B000000u, 0x7440 + b));
+						half_stage(v[b]);
 					}
+					put(u, v);
 				}
-				put(pr, v);
 			}
 			if (!buf.tile_done)
 				pdl_wait(); // before this level's stores
@@ -699,18 +726,29 @@ __device__ __forceinline__ void dwt_forward_body(DwtSharedT<DwtSplit<kThreads, k
 		{
 			const LevelDesc &P = p.P;
 			const int64_t ll = comp == 0 ? p.prev_ll[0] : (comp == 1 ? p.prev_ll[1] : p.prev_ll[2]);
-			const bool f16 = P.fp16 != 0;
+			const bool f16 = kHalf && P.fp16 != 0;
 			float4 raw[kIters][2];
+			if (interior && !f16)
+			{
+				const float *at = buf.coef32 + ll + int64_t(y0 + pr0) * P.pitch + x;
 #pragma unroll
-			for (int u = 0; u < kIters; u++)
+				for (int u = 0; u < kIters; u++)
 #pragma unroll
-				for (int h = 0; h < 2; h++)
-				{
-					const int pr = pr0 + u * kLoadRows;
-					raw[u][h] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-					if (loader && pr < kPairRows)
+					for (int h = 0; h < 2; h++)
+						raw[u][h] = __ldcg(reinterpret_cast<const float4 *>(
+						    at + (pair_row(u) - pr0 + h * kPairRows) * P.pitch));
+			}
+			else
+			{
+				int4 xi = make_int4(x, x + 1, x + 2, x + 3);
+				if (!inside)
+					xi = *reinterpret_cast<const int4 *>(&sh.xidx[4 * j]);
+#pragma unroll
+				for (int u = 0; u < kIters; u++)
+#pragma unroll
+					for (int h = 0; h < 2; h++)
 					{
-						const int64_t row = ll + int64_t(row_of(pr + h * kPairRows)) * P.pitch;
+						const int64_t row = ll + int64_t(row_of(pair_row(u) + h * kPairRows)) * P.pitch;
 						if (!inside)
 							raw[u][h] = make_float4(load_coef(buf.coef32, buf.coef16, f16, row + xi.x),
 							                        load_coef(buf.coef32, buf.coef16, f16, row + xi.y),
@@ -718,24 +756,21 @@ __device__ __forceinline__ void dwt_forward_body(DwtSharedT<DwtSplit<kThreads, k
 							                        load_coef(buf.coef32, buf.coef16, f16, row + xi.w));
 						else if (f16)
 						{
-							const uint2 hv = __ldcg(reinterpret_cast<const uint2 *>(buf.coef16 + row + xi.x));
+							const uint2 hv = __ldcg(reinterpret_cast<const uint2 *>(buf.coef16 + row + x));
 							const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&hv.x));
 							const float2 b = __half22float2(*reinterpret_cast<const __half2 *>(&hv.y));
 							raw[u][h] = make_float4(a.x, a.y, b.x, b.y);
 						}
 						else
-							raw[u][h] = __ldcg(reinterpret_cast<const float4 *>(buf.coef32 + row + xi.x));
+							raw[u][h] = __ldcg(reinterpret_cast<const float4 *>(buf.coef32 + row + x));
 					}
-				}
+			}
 #pragma unroll
 			for (int u = 0; u < kIters; u++)
 			{
-				const int pr = pr0 + u * kLoadRows;
-				if (!loader || pr >= kPairRows)
-					continue;
 				const f32x2 v[4] = {f2_pack(raw[u][0].x, raw[u][1].x), f2_pack(raw[u][0].y, raw[u][1].y),
 				                    f2_pack(raw[u][0].z, raw[u][1].z), f2_pack(raw[u][0].w, raw[u][1].w)};
-				put(pr, v);
+				put(u, v);
 			}
 		}
 	}
@@ -777,7 +812,7 @@ __device__ __forceinline__ void dwt_forward_body(DwtSharedT<DwtSplit<kThreads, k
 					f2_unpack(e[5 + 2 * (k + m)], a, b);
 					hi0[m] = __fmul_rn(a, kK);
 					hi1[m] = __fmul_rn(b, kK);
-					if (L.stage16)
+					if (kHalf && L.stage16)
 					{
 						lo0[m] = round_to_half(lo0[m]);
 						lo1[m] = round_to_half(lo1[m]);
@@ -809,49 +844,63 @@ __device__ __forceinline__ void dwt_forward_body(DwtSharedT<DwtSplit<kThreads, k
 			for (int j = 0; j < kWin; j++)
 				e[j] = *reinterpret_cast<const f32x2 *>(&sh.h[seg * 2 * kPairs + j][col]);
 			lift_forward2(e);
-			const int c = col & 31;
-			const int b_low = col < 32 ? 0 : 1;
-			const int gx = tx * 32 + c;
-			const int r0 = stripe * kRows + seg * kPairs;
-			const int64_t at = int64_t(ty * 32 + r0) * L.pitch + gx;
+			const int c = col & 31, b_low = col >> 5;
+			const int gx = tx * 32 + c, gy = ty * 32 + stripe * kRows + seg * kPairs;
+			const int64_t at = int64_t(gy) * L.pitch + gx;
 			const int64_t at_low = p.band[comp][b_low].offset + at, at_high = p.band[comp][b_low + 2].offset + at;
 #pragma unroll
 			for (int k = 0; k < kPairs; k++)
 			{
-				f32x2 lo = f2_mul_rn(e[4 + 2 * k], f2_pack(kInvK, kInvK)), hi = f2_mul_rn(e[5 + 2 * k], f2_pack(kK, kK));
-				if (!whole || L.fp16 || L.stage16)
-				{
-					float a[4];
-					f2_unpack(lo, a[0], a[1]);
-					f2_unpack(hi, a[2], a[3]);
+				e[4 + 2 * k] = f2_mul_rn(e[4 + 2 * k], f2_pack(kInvK, kInvK));
+				e[5 + 2 * k] = f2_mul_rn(e[5 + 2 * k], f2_pack(kK, kK));
+			}
+			if (!whole || (kHalf && (L.fp16 || L.stage16)))
+			{
 #pragma unroll
-					for (int i = 0; i < 4; i++)
+				for (int k = 0; k < 2 * kPairs; k++)
+				{
+					float a[2];
+					f2_unpack(e[4 + k], a[0], a[1]);
+#pragma unroll
+					for (int i = 0; i < 2; i++)
 					{
-						if (L.fp16 || L.stage16)
+						if (kHalf && (L.fp16 || L.stage16))
 							a[i] = round_to_half(a[i]);
-						if (gx + (i & 1) >= L.width || ty * 32 + r0 + k >= L.height)
+						if (gx + i >= L.width || gy + (k >> 1) >= L.height)
 							a[i] = 0.0f;
 					}
-					lo = f2_pack(a[0], a[1]);
-					hi = f2_pack(a[2], a[3]);
+					e[4 + k] = f2_pack(a[0], a[1]);
 				}
-				if (L.fp16)
+			}
+			if (kHalf && L.fp16)
+			{
+#pragma unroll
+				for (int k = 0; k < kPairs; k++)
 				{
 					float a[4];
-					f2_unpack(lo, a[0], a[1]);
-					f2_unpack(hi, a[2], a[3]);
+					f2_unpack(e[4 + 2 * k], a[0], a[1]);
+					f2_unpack(e[5 + 2 * k], a[2], a[3]);
 					*reinterpret_cast<__half2 *>(buf.coef16 + at_low + k * L.pitch) = __floats2half2_rn(a[0], a[1]);
 					*reinterpret_cast<__half2 *>(buf.coef16 + at_high + k * L.pitch) = __floats2half2_rn(a[2], a[3]);
 				}
-				else
+			}
+			else
+			{
+				float *low = buf.coef32 + at_low, *high = buf.coef32 + at_high;
+#pragma unroll
+				for (int k = 0; k < kPairs; k++, low += L.pitch, high += L.pitch)
 				{
-					*reinterpret_cast<f32x2 *>(buf.coef32 + at_low + k * L.pitch) = lo;
-					*reinterpret_cast<f32x2 *>(buf.coef32 + at_high + k * L.pitch) = hi;
+					*reinterpret_cast<f32x2 *>(low) = e[4 + 2 * k];
+					*reinterpret_cast<f32x2 *>(high) = e[5 + 2 * k];
 				}
-				if (kStripes == 1 && fused)
+			}
+			if constexpr (kStripes == 1)
+			{
+#pragma unroll
+				for (int k = 0; k < kPairs; k++)
 				{
-					*reinterpret_cast<f32x2 *>(&sh.bands[b_low][r0 + k][c]) = lo;
-					*reinterpret_cast<f32x2 *>(&sh.bands[b_low + 2][r0 + k][c]) = hi;
+					*reinterpret_cast<f32x2 *>(&sh.bands[b_low][seg * kPairs + k][c]) = e[4 + 2 * k];
+					*reinterpret_cast<f32x2 *>(&sh.bands[b_low + 2][seg * kPairs + k][c]) = e[5 + 2 * k];
 				}
 			}
 		}
@@ -869,12 +918,12 @@ __device__ __forceinline__ void dwt_forward_body(DwtSharedT<DwtSplit<kThreads, k
 	}
 }
 
-template <int kThreads>
+template <int kThreads, bool kHalf>
 __global__ void __launch_bounds__(kThreads, DwtSplit<kThreads, 1>::kMinBlocks)
     dwt_forward_kernel(const LevelParams p, const PlaneInput in, const EncodeBuffers buf, const int fused)
 {
 	__shared__ DwtShared sh;
-	dwt_forward_body<kThreads>(sh, p, in, buf, fused, int(blockIdx.x), int(blockIdx.y));
+	dwt_forward_body<kThreads, 1, kHalf>(sh, p, in, buf, fused, int(blockIdx.x), int(blockIdx.y));
 }
 
 // Small transform-only levels (fewer tiles than SMs): four 256-thread CTAs per
@@ -882,16 +931,17 @@ __global__ void __launch_bounds__(kThreads, DwtSplit<kThreads, 1>::kMinBlocks)
 // parameters as dwt_forward_kernel (graph nodes are updated with one argument
 // list).
 constexpr int kDwtStripes = kDwtStripeCtas;
+template <bool kHalf>
 __global__ void __launch_bounds__(kLargeLevelThreads, 4)
     dwt_stripes_kernel(const LevelParams p, const PlaneInput in, const EncodeBuffers buf, const int fused)
 {
 	(void)fused;
 	__shared__ DwtSharedT<DwtSplit<kLargeLevelThreads, kDwtStripes>::kRowsIn> sh;
-	dwt_forward_body<kLargeLevelThreads, kDwtStripes>(sh, p, in, buf, 0, int(blockIdx.x) / kDwtStripes, int(blockIdx.y),
-	                                                  int(blockIdx.x) % kDwtStripes);
+	dwt_forward_body<kLargeLevelThreads, kDwtStripes, kHalf>(sh, p, in, buf, 0, int(blockIdx.x) / kDwtStripes,
+	                                                         int(blockIdx.y), int(blockIdx.x) % kDwtStripes);
 }
 
-// Batched form: one CTA per (frame, component, tile) of this level.
+// Batched form (FP32 storage): one CTA per (frame, component, tile) of this level.
 template <int kThreads>
 __global__ void __launch_bounds__(kThreads, DwtSplit<kThreads, 1>::kMinBlocks)
     dwt_forward_batch_kernel(const BatchFrame *frames, const BatchFrameIO *io, const uint32_t *cta_map, const int level,
@@ -908,7 +958,7 @@ __global__ void __launch_bounds__(kThreads, DwtSplit<kThreads, 1>::kMinBlocks)
 	__syncthreads();
 	const int ntiles = s_p.L.tiles_x * s_p.L.tiles_y;
 	__shared__ DwtShared sh;
-	dwt_forward_body<kThreads>(sh, s_p, s_in, s_buf, fused, local % ntiles, local / ntiles);
+	dwt_forward_body<kThreads, 1, false>(sh, s_p, s_in, s_buf, fused, local % ntiles, local / ntiles);
 }
 
 // Quantiser over a pyramid already in storage (the reference's
@@ -1834,8 +1884,8 @@ __device__ __noinline__ void batch_forward_item(int level, int small_level, int 
 {
 	BatchShared &sh = batch_shared();
 	const int per_comp = sh.prm.lp.L.tiles_x * sh.prm.lp.L.tiles_y;
-	dwt_forward_body<kBatchPersistentThreads>(sh.u.dwt, sh.prm.lp, sh.in, sh.eb, level < small_level ? 1 : 0,
-	                                          local % per_comp, local / per_comp);
+	dwt_forward_body<kBatchPersistentThreads, 1, false>(sh.u.dwt, sh.prm.lp, sh.in, sh.eb, level < small_level ? 1 : 0,
+	                                                    local % per_comp, local / per_comp);
 }
 
 __device__ __noinline__ void batch_quant_item(int small_blocks, int local)
@@ -1866,7 +1916,7 @@ __device__ __noinline__ void batch_inverse_item(int local)
 {
 	BatchShared &sh = batch_shared();
 	const int per_comp = sh.prm.lp.L.tiles_x * sh.prm.lp.L.tiles_y;
-	idwt_body<kBatchPersistentThreads>(sh.u.idwt, sh.prm.lp, sh.di, sh.out, nullptr, local % per_comp,
+	idwt_body<kBatchPersistentThreads, 1, false>(sh.u.idwt, sh.prm.lp, sh.di, sh.out, nullptr, local % per_comp,
 	                                   local / per_comp);
 }
 
@@ -2026,20 +2076,17 @@ void launch_dwt_forward_level(const LevelParams &p, const PlaneInput &in, const 
 {
 	const dim3 grid(p.L.tiles_x * p.L.tiles_y, (p.level == 0 && !p.chroma444) ? 1 : 3);
 	const int f = forward_fused_mode(p, fused_quant);
+	const bool half = p.L.fp16 || p.L.stage16 || (p.level > 0 && p.P.fp16);
 	if (int(grid.x * grid.y) < kSmallLevelTiles && f == 0)
 	{
 		LaunchConfig lc(dim3(grid.x * kDwtStripes, grid.y), dim3(kLargeLevelThreads), stream, programmatic);
-		cudaLaunchKernelEx(&lc.cfg, dwt_stripes_kernel, p, in, buf, f);
-	}
-	else if (int(grid.x * grid.y) < kSmallLevelTiles)
-	{
-		LaunchConfig lc(grid, dim3(1024), stream, programmatic);
-		cudaLaunchKernelEx(&lc.cfg, dwt_forward_kernel<1024>, p, in, buf, f);
+		cudaLaunchKernelEx(&lc.cfg, half ? dwt_stripes_kernel<true> : dwt_stripes_kernel<false>, p, in, buf, f);
 	}
 	else
 	{
 		LaunchConfig lc(grid, dim3(kLargeLevelThreads), stream, programmatic);
-		cudaLaunchKernelEx(&lc.cfg, dwt_forward_kernel<kLargeLevelThreads>, p, in, buf, f);
+		cudaLaunchKernelEx(&lc.cfg, half ? dwt_forward_kernel<kLargeLevelThreads, true> : dwt_forward_kernel<kLargeLevelThreads, false>,
+		                   p, in, buf, f);
 	}
 }
 
