@@ -141,16 +141,22 @@ __device__ __forceinline__ bool wait_counter(const uint32_t *c, uint32_t target)
 	return true;
 }
 
+// GPU-scope release increment: what this thread stored, or observed through a
+// CTA barrier, is visible to whoever acquires the counter's new value.
+__device__ __forceinline__ void red_release_add(uint32_t *c, uint32_t v)
+{
+	asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(c), "r"(v) : "memory");
+}
+
 // Adds one to a counter once every thread of the CTA has stored its part
 // (called by every thread; the barrier orders the CTA's stores before the
-// fence of thread 0).
+// release of one thread of the last warp, which has the least left to do).
 __device__ __forceinline__ void cta_count_done(uint32_t *c)
 {
 	__syncthreads();
-	if (threadIdx.x == 0)
+	if (threadIdx.x == blockDim.x - 32)
 	{
-		__threadfence();
-		atomicAdd(c, 1u);
+		red_release_add(c, 1u);
 	}
 }
 

@@ -387,14 +387,14 @@ BlockParams make_block_params(const Geometry &g)
 // transform tile), components and tiles in order within a level. Fills in the
 // counters' offsets and the count at which each level's tiles are complete
 // (the CTAs storing one tile: row stripes for the small transform-only levels,
-// as launch_dwt_forward_level launches them), and the number of 32x32 blocks
-// the forward levels quantise themselves. Returns the number of counters.
+// as launch_dwt_forward_level launches them), and the number of forward-level
+// CTAs with a fused quantiser. Returns the number of counters.
 int setup_tile_dataflow(const Geometry &g, int small_level, LevelParams (&lp)[kLevels], BlockParams &bp,
-                        uint32_t &fused_blocks)
+                        uint32_t &fused_ctas)
 {
 	int32_t offset[kLevels] = {}, parts[kLevels] = {};
 	int total = 0;
-	fused_blocks = 0;
+	fused_ctas = 0;
 	for (int level = 0; level < kLevels; level++)
 	{
 		const int comps = (level == 0 && !g.chroma444) ? 1 : kComponents;
@@ -404,7 +404,7 @@ int setup_tile_dataflow(const Geometry &g, int small_level, LevelParams (&lp)[kL
 		const bool transform_only = level >= small_level;
 		parts[level] = (transform_only && tiles < kSmallLevelTiles) ? kDwtStripeCtas : 1;
 		if (!transform_only)
-			fused_blocks += uint32_t(tiles) * (level == kLevels - 1 ? 4u : 3u);
+			fused_ctas += uint32_t(tiles);
 	}
 	for (int level = 0; level < kLevels; level++)
 	{
@@ -736,7 +736,7 @@ struct pyrowave_encoder_opaque
 	// Tile dataflow of the captured encode: counters right after the rate-control
 	// state in the same allocation (one clear covers both).
 	int tile_counters = 0;
-	uint32_t fused_blocks = 0;
+	uint32_t fused_ctas = 0;
 	// Packing analysis (allocated by its first call): the 64x64 region table and
 	// the device accumulators.
 	int32_t *analysis_regions = nullptr;
@@ -830,7 +830,7 @@ struct pyrowave_encoder_opaque
 			lp[level] = make_level_params(g, level);
 		bp = make_block_params(g);
 		small_level_split(g, small_level, small_blocks);
-		tile_counters = setup_tile_dataflow(g, small_level, lp, bp, fused_blocks);
+		tile_counters = setup_tile_dataflow(g, small_level, lp, bp, fused_ctas);
 		(void)resolve_cluster_max();
 		bool ok = true;
 		coef32 = dev_alloc<float>(size_t(g.storage_elems32), ok);
@@ -915,7 +915,7 @@ struct pyrowave_encoder_opaque
 	ResolveParams dataflow_resolve_params(uint32_t target_words) const
 	{
 		ResolveParams rp = make_resolve_params(g, target_words, sequence_count);
-		rp.fused_blocks = fused_blocks;
+		rp.fused_ctas = fused_ctas;
 		return rp;
 	}
 

@@ -133,7 +133,7 @@ struct RateControlState
 	int32_t xstar;                 // first partially applied bucket*16+subdivision (-1 none)
 	uint32_t sequence;
 	uint32_t decode_error;         // kDecodeError* bits of the batched form's decode of this frame
-	uint32_t fused_done;           // tile dataflow: blocks quantised by the forward levels
+	uint32_t fused_done;           // tile dataflow: forward-level CTAs whose quantiser finished
 	// Per resolve slice: words << 32 | non-empty blocks << 1 | 1 once published.
 	unsigned long long slice_total[kMaxResolveSlices];
 };
@@ -298,7 +298,7 @@ struct ResolveParams
 	int32_t block_count_32x32, blocks_per_subdivision, subdivision_shift;
 	int32_t width, height, chroma444;
 	uint32_t target_words, sequence;
-	uint32_t fused_blocks; // tile dataflow: blocks quantised by the forward levels, to wait for (0: none)
+	uint32_t fused_ctas; // tile dataflow: forward-level CTAs with a fused quantiser, to wait for (0: none)
 };
 
 // cudaLaunchKernelEx configuration, optionally marked as a programmatic
