@@ -291,6 +291,14 @@ __device__ __forceinline__ void st_cluster_u64(const void *local_smem, uint32_t 
 	asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(remote), "l"(v) : "memory");
 }
 
+// Eight floats as one 32-byte store (32-byte aligned).
+__device__ __forceinline__ void store_f32x8(float *p, float a, float b, float c, float d, float e, float f, float g, float h)
+{
+	asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d), "f"(e),
+	             "f"(f), "f"(g), "f"(h)
+	             : "memory");
+}
+
 // 8x8 bit-matrix transpose: bit j of byte i of the input becomes bit i of byte
 // j of the output (three swap stages of 1, 2 and 4 bit-square blocks).
 __device__ __forceinline__ unsigned long long transpose8x8(unsigned long long x)
