@@ -448,9 +448,9 @@ __device__ __forceinline__ void compute_quant_scale_any(float max_wave, uint32_t
 // that. So the rounded quotient compares with (code + 2) / 8 as the exact one
 // does, and code + 2 = k is the smallest integer with 8 max <= target * k: an
 // estimate that is k or k - 1, then one exact comparison. A maximum below 1 has
-// k = 8.
+// k = 8. Returns k; the scale is 8 / k.
 constexpr float kQuantScaleFast = 262144.0f;
-__device__ __forceinline__ void compute_quant_scale(float max_wave, uint32_t &code, float &scale)
+__device__ __forceinline__ int quant_scale_step(float max_wave)
 {
 	const int e = int(__float_as_uint(__fsub_rn(max_wave, 0.25f)) >> 23) - 126;
 	const float target4 = __fsub_rn(__int_as_float((e + 129) << 23), 1.0f), max32 = __fmul_rn(max_wave, 32.0f);
@@ -459,10 +459,7 @@ __device__ __forceinline__ void compute_quant_scale(float max_wave, uint32_t &co
 	float k = ceilf(__fmul_rn(__fmul_rn(max32, r), 1.0f - 0x1p-21f));
 	if (max32 > __fmul_rn(target4, k))
 		k = __fadd_rn(k, 1.0f);
-	if (max_wave < 1.0f)
-		k = 8.0f;
-	code = uint32_t(int(k)) - 2u;
-	scale = __frcp_rn(__fmul_rn(k, 0.125f));
+	return max_wave < 1.0f ? 8 : int(k);
 }
 
 // Sum over the eight plane codes p of cw of max(p - d, 0), d = 0, 1 or 2.

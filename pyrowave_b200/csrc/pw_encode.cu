@@ -61,10 +61,27 @@ __device__ __forceinline__ float max3_nan(float a, float b, float c)
 // Position of the highest set bit of int(x), x in [0, 32767] (-1: none), from the exponent.
 __device__ __forceinline__ int float_msb(float x) { return max(int(__float_as_uint(x) >> 23) - 127, -1); }
 
+// Per scale code, by k = code + 2: the 8x8 scale 8 / k and the squared inverse
+// of the band's quantiser with it, computed once per band tile (k is at most 14
+// below kQuantScaleFast). Threads 0..15 of a group fill it.
+struct QuantScales
+{
+	float2 by_k[16];
+};
+__device__ __forceinline__ float2 quant_scale_entry(float scale, float quant_resolution)
+{
+	const float inv_quant = __frcp_rn(__fmul_rn(quant_resolution, scale));
+	return make_float2(scale, __fmul_rn(inv_quant, inv_quant));
+}
+__device__ __forceinline__ void fill_quant_scales(QuantScales &sc, int k, float quant_resolution)
+{
+	sc.by_k[k] = quant_scale_entry(__frcp_rn(__fmul_rn(float(max(k, 1)), 0.125f)), quant_resolution);
+}
+
 template <int S>
 __device__ __forceinline__ void quant_analyze_row(const float *tile, const int ly, const int r, QuantGroupShared &sh,
-                                                  const LevelDesc &L, const BandParam &B, const int bx32,
-                                                  const int by32, const EncodeBuffers &buf)
+                                                  const QuantScales &scales, const LevelDesc &L, const BandParam &B,
+                                                  const int bx32, const int by32, const EncodeBuffers &buf)
 {
 	const unsigned full = 0xffffffffu;
 	const int lane = threadIdx.x & 31;
@@ -73,24 +90,37 @@ __device__ __forceinline__ void quant_analyze_row(const float *tile, const int l
 	const bool in_range = x8 < L.blocks8_x && y8 < L.blocks8_y;
 	const float qres = B.quant_resolution;
 
-	float4 row0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), row1 = row0;
-	if (in_range)
-	{
-		const float *src = tile + (ly * 8 + sub_y(sub)) * kBandPitch + lx * 8 + sub_x(sub);
-		row0 = *reinterpret_cast<const float4 *>(src);
-		row1 = *reinterpret_cast<const float4 *>(src + kBandPitch);
-	}
-	float v[8] = {__fmul_rn(row0.x, qres), __fmul_rn(row1.x, qres), __fmul_rn(row0.y, qres), __fmul_rn(row1.y, qres),
-	              __fmul_rn(row0.z, qres), __fmul_rn(row1.z, qres), __fmul_rn(row0.w, qres), __fmul_rn(row1.w, qres)};
+	// Samples beyond the band are zeros in the tile.
+	const float *src = tile + (ly * 8 + sub_y(sub)) * kBandPitch + lx * 8 + sub_x(sub);
+	const ulonglong2 row0 = *reinterpret_cast<const ulonglong2 *>(src);
+	const ulonglong2 row1 = *reinterpret_cast<const ulonglong2 *>(src + kBandPitch);
+	// Coefficient i = 2 * column + row of the sub-block: pairs (0, 2), (4, 6) and
+	// (1, 3), (5, 7) of the two rows.
+	const f32x2 qres2 = f2_pack(qres, qres);
+	const f32x2 vp[4] = {f2_mul_rn(row0.x, qres2), f2_mul_rn(row0.y, qres2), f2_mul_rn(row1.x, qres2),
+	                     f2_mul_rn(row1.y, qres2)};
+	float v[8];
+	f2_unpack(vp[0], v[0], v[2]);
+	f2_unpack(vp[1], v[4], v[6]);
+	f2_unpack(vp[2], v[1], v[3]);
+	f2_unpack(vp[3], v[5], v[7]);
 
-	// 8x8 maximum and quant scale (wavelet_quant.comp:174-181). The maximum
-	// ignores NaN, and a NaN value is clamped to -32767 below.
+	// 8x8 maximum and quant scale (wavelet_quant.comp:174-181).
 	float max_sub = max3_nan(fabsf(v[0]), fabsf(v[1]), fabsf(v[2]));
 	max_sub = max3_nan(max_sub, fabsf(v[3]), fabsf(v[4]));
 	max_sub = max3_nan(max_sub, fabsf(v[5]), fabsf(v[6]));
 	max_sub = max3_nan(max_sub, fabsf(v[7]), 0.0f);
-	if (max_sub != max_sub)
+	float max_wave = max_sub;
+	max_wave = max3_nan(max_wave, __shfl_xor_sync(full, max_wave, 1), 0.0f);
+	max_wave = max3_nan(max_wave, __shfl_xor_sync(full, max_wave, 2), 0.0f);
+	max_wave = max3_nan(max_wave, __shfl_xor_sync(full, max_wave, 4), 0.0f);
+
+	uint32_t qcode;
+	float qs, iqs;
+	if (__any_sync(full, !(max_wave < kQuantScaleFast)))
 	{
+		// A value too large for the short form of the scale, or NaN: the maximum
+		// ignores NaN, and a NaN value is clamped to -32767 below.
 		max_sub = 0.0f;
 #pragma unroll
 		for (int i = 0; i < 8; i++)
@@ -98,39 +128,64 @@ __device__ __forceinline__ void quant_analyze_row(const float *tile, const int l
 			max_sub = fmaxf(max_sub, fabsf(v[i]));
 			v[i] = v[i] != v[i] ? -3.0e38f : v[i];
 		}
-	}
-	float max_wave = max_sub;
-	max_wave = fmaxf(max_wave, __shfl_xor_sync(full, max_wave, 1));
-	max_wave = fmaxf(max_wave, __shfl_xor_sync(full, max_wave, 2));
-	max_wave = fmaxf(max_wave, __shfl_xor_sync(full, max_wave, 4));
-
-	uint32_t qcode;
-	float qs;
-	if (__any_sync(full, max_wave >= kQuantScaleFast))
+		max_wave = max_sub;
+		max_wave = fmaxf(max_wave, __shfl_xor_sync(full, max_wave, 1));
+		max_wave = fmaxf(max_wave, __shfl_xor_sync(full, max_wave, 2));
+		max_wave = fmaxf(max_wave, __shfl_xor_sync(full, max_wave, 4));
 		compute_quant_scale_any(max_wave, qcode, qs);
+		iqs = quant_scale_entry(qs, qres).y;
+	}
 	else
-		compute_quant_scale(max_wave, qcode, qs);
+	{
+		const int k = quant_scale_step(max_wave);
+		qcode = uint32_t(k - 2);
+		const float2 e = scales.by_k[k];
+		qs = e.x;
+		iqs = e.y;
+	}
+	const f32x2 qs2 = f2_pack(qs, qs);
+#pragma unroll
+	for (int i = 0; i < 4; i++)
+	{
+		// Pairs (i, i + 4): adjacent as the two packed products leave them free.
+		f32x2 p = f2_mul_rn(f2_pack(v[i], v[i + 4]), qs2);
+		f2_unpack(p, v[i], v[i + 4]);
+	}
 	float av[8];
 #pragma unroll
 	for (int i = 0; i < 8; i++)
-	{
-		v[i] = __fmul_rn(v[i], qs);
 		av[i] = fminf(fabsf(v[i]), kMaxScaledMagnitude);
-	}
 	max_sub = fminf(__fmul_rn(max_sub, qs), kMaxScaledMagnitude);
 	max_wave = fminf(__fmul_rn(max_wave, qs), kMaxScaledMagnitude);
 	const int msb = float_msb(max_wave);
 	const int warp_msb = __reduce_max_sync(full, msb);
+	// Magnitudes as pairs (i, i + 4): the two lanes of a pair accumulate the two
+	// halves of the squared error, over i = 0..3 and i = 4..7, in the same order
+	// as eight scalar steps would.
+	f32x2 avp[4];
+#pragma unroll
+	for (int j = 0; j < 4; j++)
+		avp[j] = f2_pack(av[j], av[j + 4]);
 
 	// The packer's input: the scaled values as sign-magnitude (|int(v)| <= 32767),
 	// one 16-byte store per sub-block, written by the first warp of each row.
 	// int(|v|) is the low half of |v| + 2^23 rounded toward zero; the sign of a
 	// magnitude of zero is not read.
 	uint32_t mag[4];
+	{
+		uint32_t m[8];
 #pragma unroll
-	for (int j = 0; j < 4; j++)
-		mag[j] = __byte_perm(__float_as_uint(__fadd_rz(av[2 * j], 8388608.0f)),
-		                     __float_as_uint(__fadd_rz(av[2 * j + 1], 8388608.0f)), 0x5410);
+		for (int j = 0; j < 4; j++)
+		{
+			float lo, hi;
+			f2_unpack(f2_add_rz(avp[j], f2_pack(8388608.0f, 8388608.0f)), lo, hi);
+			m[j] = __float_as_uint(lo);
+			m[j + 4] = __float_as_uint(hi);
+		}
+#pragma unroll
+		for (int j = 0; j < 4; j++)
+			mag[j] = __byte_perm(m[2 * j], m[2 * j + 1], 0x5410);
+	}
 	if (r == 0 && buf.mag16)
 	{
 		uint32_t w[4];
@@ -158,9 +213,6 @@ __device__ __forceinline__ void quant_analyze_row(const float *tile, const int l
 		return;
 	}
 
-	const float overall = __fmul_rn(qres, qs);
-	const float inv_quant = __frcp_rn(overall);
-	const float iqs = __fmul_rn(inv_quant, inv_quant);
 	const float rdo = B.rdo_scale;
 
 	// Stats at q = 0 (wavelet_quant.comp:139-165,205-238): the 8x8's plane codes
@@ -176,14 +228,6 @@ __device__ __forceinline__ void quant_analyze_row(const float *tile, const int l
 	codes += __shfl_xor_sync(full, codes, 2);
 	codes += __shfl_xor_sync(full, codes, 4);
 	const uint32_t nsig0 = codes >> 16;
-
-	// Magnitudes as pairs (i, i + 4): the two lanes of a pair accumulate the two
-	// halves of the squared error, over i = 0..3 and i = 4..7, in the same order
-	// as eight scalar steps would.
-	f32x2 avp[4];
-#pragma unroll
-	for (int j = 0; j < 4; j++)
-		avp[j] = f2_pack(av[j], av[j + 4]);
 
 	// Distortion of dropping every plane (wavelet_quant.comp:253-256).
 	float drop;
@@ -303,20 +347,21 @@ __device__ __forceinline__ void quant_analyze_row(const float *tile, const int l
 }
 
 // Rate-control row of a 32x32 block from its four rows' sums
-// (analyze_rate_control.comp:101-220): lanes 0..15 of a warp.
-__device__ __forceinline__ void quant_finish_block(const QuantGroupShared &sh, const BandParam &B,
+// (analyze_rate_control.comp:101-220), by the 16 lanes of a half-warp; every lane of
+// the warp calls it, `active` where its half has a block.
+__device__ __forceinline__ void quant_finish_block(const bool active, const QuantGroupShared &sh, const BandParam &B,
                                                    const int subdivision_shift, const int bx32, const int by32,
                                                    const EncodeBuffers &buf)
 {
-	const int i = threadIdx.x & 31;
+	const int i = threadIdx.x & 15;
 	const float d = __fadd_rn(__fadd_rn(sh.dist[0][i], sh.dist[1][i]), __fadd_rn(sh.dist[2][i], sh.dist[3][i]));
 	uint32_t c = sh.cost[0][i] + sh.cost[1][i] + sh.cost[2][i] + sh.cost[3][i];
 	if (c != 0)
 		c += 64;
 	const uint32_t rate = (c + 31) >> 5;
-	const unsigned m16 = 0x0000ffffu;
-	const float d0 = __shfl_sync(m16, d, 0);
-	const uint32_t r0 = __shfl_sync(m16, rate, 0);
+	const unsigned full = 0xffffffffu;
+	const float d0 = __shfl_sync(full, d, 0, 16);
+	const uint32_t r0 = __shfl_sync(full, rate, 0, 16);
 	uint32_t bk = bucket_index(d, float(rate), d0, float(r0));
 	if (i == 0)
 		bk = 0;
@@ -325,11 +370,13 @@ __device__ __forceinline__ void quant_finish_block(const QuantGroupShared &sh, c
 #pragma unroll
 	for (int off = 1; off < 16; off *= 2)
 	{
-		const uint32_t up = __shfl_up_sync(m16, bk, off) + uint32_t(off);
+		const uint32_t up = __shfl_up_sync(full, bk, off, 16) + uint32_t(off);
 		if (i >= off)
 			bk = max(bk, up);
 	}
-	const uint32_t rate_prev = __shfl_up_sync(m16, rate, 1);
+	const uint32_t rate_prev = __shfl_up_sync(full, rate, 1, 16);
+	if (!active)
+		return;
 	const uint32_t block_index = uint32_t(B.block32_offset + by32 * B.block32_stride + bx32);
 	buf.rd_cost[block_index * 16 + i] = uint16_t(rate);
 	buf.rd_bucket[block_index * 16 + i] = uint8_t(bk);
@@ -371,6 +418,7 @@ template <int kRowsIn> struct DwtSharedT
 	};
 	alignas(16) float h[kRowsIn][kHPitch]; // after horizontal lifting: low in 0..31, high in 32..63
 	QuantGroupShared q[4];
+	QuantScales scales[4]; // of the bands the tile's quantiser codes
 };
 
 // Work split of the forward level for a CTA of kThreads threads. Whole tiles
@@ -489,7 +537,7 @@ __device__ __forceinline__ void quant_tile(DwtShared &sh, const LevelParams &p, 
 		split_tail = fused == kFusedSplitTail && (nb % Split::kGroups) != 0;
 	const int rounds = split_tail ? nb / Split::kGroups : (nb + Split::kGroups - 1) / Split::kGroups;
 	for (int bi = grp; bi < min(nb, rounds * Split::kGroups); bi += Split::kGroups)
-		quant_analyze_row<Split::kQSplit>(&sh.bands[first_band + bi][0][0], ly, t >> 7, sh.q[bi], L,
+		quant_analyze_row<Split::kQSplit>(&sh.bands[first_band + bi][0][0], ly, t >> 7, sh.q[bi], sh.scales[bi], L,
 		                                  p.band[comp][first_band + bi], tx, ty, buf);
 	if constexpr (kThreads == kLargeLevelThreads)
 	{
@@ -497,21 +545,21 @@ __device__ __forceinline__ void quant_tile(DwtShared &sh, const LevelParams &p, 
 		{
 			const int bi = rounds * Split::kGroups;
 			quant_analyze_row<2 * Split::kQSplit>(&sh.bands[first_band + bi][0][0], ly, int(threadIdx.x) >> 7, sh.q[bi],
-			                                      L, p.band[comp][first_band + bi], tx, ty, buf);
+			                                      sh.scales[bi], L, p.band[comp][first_band + bi], tx, ty, buf);
 		}
 	}
 	__syncthreads();
-	// One warp per band finishes its block. Tile dataflow: the resolve waits for
+	// A half-warp per band finishes its block. Tile dataflow: the resolve waits for
 	// the count of every CTA, released once after all of its bands' rows (a full
 	// fence and count per band cost 4 us of a 4K 4:4:4 frame's encode).
-	const int bi = int(threadIdx.x) >> 5;
-	if (bi >= nb)
+	const int bi = int(threadIdx.x) >> 4;
+	if ((bi & ~1) >= nb)
 		return;
-	if ((threadIdx.x & 31) < 16)
-		quant_finish_block(sh.q[bi], p.band[comp][first_band + bi], p.subdivision_shift, tx, ty, buf);
+	quant_finish_block(bi < nb, sh.q[min(bi, nb - 1)], p.band[comp][first_band + min(bi, nb - 1)], p.subdivision_shift, tx, ty,
+	                   buf);
 	if (buf.tile_done)
 	{
-		asm volatile("bar.sync 1, %0;" ::"r"(32 * nb) : "memory");
+		asm volatile("bar.sync 1, 64;" ::: "memory"); // the two finishing warps
 		if (threadIdx.x == 0)
 			red_release_add(&buf.rc->fused_done, 1u);
 	}
@@ -772,6 +820,13 @@ __device__ __forceinline__ void dwt_forward_body(DwtSharedT<DwtSplit<kThreads, k
 	}
 	__syncthreads();
 
+	if (kStripes == 1 && fused && threadIdx.x >= kThreads - 64)
+	{
+		// The last two warps have the lightest load below.
+		const int i = int(threadIdx.x) - (kThreads - 64), first_band = level == kLevels - 1 ? 0 : 1;
+		if (first_band + (i >> 4) < 4)
+			fill_quant_scales(sh.scales[i >> 4], i & 15, p.band[comp][first_band + (i >> 4)].quant_resolution);
+	}
 	// Horizontal lifting of row pairs, segments of kHPairs output pairs. Items
 	// start at another warp from tile to tile: they fill half the warps, and
 	// warps of one index share an issue port.
@@ -965,7 +1020,7 @@ __global__ void __launch_bounds__(kThreads, DwtSplit<kThreads, 1>::kMinBlocks)
 template <int S, int G>
 __device__ __forceinline__ void quant_blocks_body(const BlockParams &p, const EncodeBuffers &buf, const int first,
                                                   const int end, const int item, float (*tile)[32][kBandPitch],
-                                                  QuantGroupShared *q)
+                                                  QuantGroupShared *q, QuantScales *scales)
 {
 	constexpr int kGroupThreads = 128 * S;
 	pdl_trigger();
@@ -986,6 +1041,8 @@ __device__ __forceinline__ void quant_blocks_body(const BlockParams &p, const En
 	}
 	else
 		pdl_wait();
+	if (active && t < 16)
+		fill_quant_scales(scales[grp], t, E.quant_resolution);
 	if (active)
 	{
 		// The block's 32 rows as 8 vectors of 4 each, every load in flight at once.
@@ -1003,6 +1060,15 @@ __device__ __forceinline__ void quant_blocks_body(const BlockParams &p, const En
 			}
 			else
 				f = __ldcg(reinterpret_cast<const float4 *>(buf.coef32 + idx));
+			// Beyond the band: zeros (storage written by the forward transform has them).
+			const int x = bx * 32 + c4, left = by * 32 + r < L.height ? L.width - x : 0;
+			if (left < 4)
+			{
+				f.x = left > 0 ? f.x : 0.0f;
+				f.y = left > 1 ? f.y : 0.0f;
+				f.z = left > 2 ? f.z : 0.0f;
+				f.w = 0.0f;
+			}
 			*reinterpret_cast<float4 *>(&tile[grp][r][c4]) = f;
 		}
 	}
@@ -1017,10 +1083,10 @@ __device__ __forceinline__ void quant_blocks_body(const BlockParams &p, const En
 	B.rdo_scale = E.rdo_scale;
 	B.quant_code = E.quant_code;
 	if (active)
-		quant_analyze_row<S>(&tile[grp][0][0], (t >> 5) & 3, t >> 7, q[grp], L, B, bx, by, buf);
+		quant_analyze_row<S>(&tile[grp][0][0], (t >> 5) & 3, t >> 7, q[grp], scales[grp], L, B, bx, by, buf);
 	__syncthreads();
-	if (active && t < 16)
-		quant_finish_block(q[grp], B, p.subdivision_shift, bx, by, buf);
+	if (t < 32)
+		quant_finish_block(active && t < 16, q[grp], B, p.subdivision_shift, bx, by, buf);
 }
 
 // One 32x32 block per CTA: the launch follows the last small-level transform
@@ -1032,7 +1098,8 @@ __global__ void __launch_bounds__(128 * S) quant_pretransformed_kernel(const Blo
 {
 	__shared__ alignas(16) float tile[1][32][kBandPitch];
 	__shared__ QuantGroupShared q[1];
-	quant_blocks_body<S, 1>(p, buf, 0, nblocks, int(blockIdx.x), tile, q);
+	__shared__ QuantScales scales[1];
+	quant_blocks_body<S, 1>(p, buf, 0, nblocks, int(blockIdx.x), tile, q, scales);
 }
 
 // Batched form: one CTA per pair of blocks among each frame's small-level blocks.
@@ -1043,12 +1110,13 @@ __global__ void __launch_bounds__(256 * S) quant_blocks_batch_kernel(const Batch
 	__shared__ EncodeBuffers s_buf;
 	__shared__ alignas(16) float tile[2][32][kBandPitch];
 	__shared__ QuantGroupShared q[2];
+	__shared__ QuantScales scales[2];
 	int f, local;
 	batch_item(cta_map, f, local);
 	load_params(s_p, frames[f].bp);
 	load_params(s_buf, frames[f].eb);
 	__syncthreads();
-	quant_blocks_body<S, 2>(s_p, s_buf, 0, frames[f].small_blocks, local, tile, q);
+	quant_blocks_body<S, 2>(s_p, s_buf, 0, frames[f].small_blocks, local, tile, q, scales);
 }
 
 // ---------------------------------------------------------------------------
@@ -1844,6 +1912,7 @@ struct BatchQuantShared
 {
 	alignas(16) float tile[2][32][kBandPitch];
 	QuantGroupShared q[2];
+	QuantScales scales[2];
 };
 
 struct BatchShared
@@ -1889,7 +1958,7 @@ __device__ __noinline__ void batch_forward_item(int level, int small_level, int 
 __device__ __noinline__ void batch_quant_item(int small_blocks, int local)
 {
 	BatchShared &sh = batch_shared();
-	quant_blocks_body<1, 2>(sh.prm.bp, sh.eb, 0, small_blocks, local, sh.u.quant.tile, sh.u.quant.q);
+	quant_blocks_body<1, 2>(sh.prm.bp, sh.eb, 0, small_blocks, local, sh.u.quant.tile, sh.u.quant.q, sh.u.quant.scales);
 }
 
 __device__ __noinline__ void batch_resolve_item(int slice, int slices)
