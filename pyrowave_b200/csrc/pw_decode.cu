@@ -60,6 +60,16 @@ __global__ void __launch_bounds__(256, 4) idwt_stripes_kernel(const LevelParams 
 	                                    int(blockIdx.x) % kIdwtStripes);
 }
 
+// Two small levels in one launch (see idwt_pair_body), grid as idwt_stripes_kernel's of the finer one.
+template <bool kHalf>
+__global__ void __launch_bounds__(256, 4) idwt_pair_kernel(const LevelParams p, const LevelParams coarser, const DecodeInput in,
+                                                           const PlaneOutput out)
+{
+	__shared__ IdwtPairShared sh;
+	idwt_pair_body<kHalf>(sh, p, coarser, in, out, int(blockIdx.x) / kIdwtStripes, int(blockIdx.y),
+	                      int(blockIdx.x) % kIdwtStripes);
+}
+
 // Batched form (FP32 storage): one CTA per (frame, component, tile) of this level.
 template <int kThreads>
 __global__ void __launch_bounds__(kThreads, kThreads >= 1024 ? 2 : 4) idwt_batch_kernel(const BatchFrame *frames, const BatchFrameIO *io,
@@ -135,6 +145,14 @@ void launch_idwt_level(const LevelParams &p, const DecodeInput &in, const PlaneO
 		LaunchConfig lc(grid, dim3(256), stream, programmatic);
 		cudaLaunchKernelEx(&lc.cfg, half ? idwt_kernel<true> : idwt_kernel<false>, p, in, out, m);
 	}
+}
+
+void launch_idwt_pair(const LevelParams &p, const LevelParams &coarser, const DecodeInput &in, const PlaneOutput &out,
+                      bool programmatic, cudaStream_t stream)
+{
+	const bool half = p.L.fp16 || p.L.stage16 || (p.level > 0 && p.P.fp16) || coarser.L.fp16;
+	LaunchConfig lc(dim3(p.L.tiles_x * p.L.tiles_y * kIdwtStripes, 3), dim3(256), stream, programmatic);
+	cudaLaunchKernelEx(&lc.cfg, half ? idwt_pair_kernel<true> : idwt_pair_kernel<false>, p, coarser, in, out);
 }
 
 void launch_pyramid_io(const BlockParams &p, float *canonical, float *coef32, __half *coef16, bool to_canonical,

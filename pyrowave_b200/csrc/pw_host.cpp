@@ -227,6 +227,12 @@ bool build_geometry(Geometry &g, std::vector<uint32_t> &jobs, int width, int hei
 	return true;
 }
 
+// Transform tiles of a level, over its components.
+int level_tiles(const Geometry &g, int level)
+{
+	return g.level[level].tiles_x * g.level[level].tiles_y * ((level == 0 && !g.chroma444) ? 1 : 3);
+}
+
 // The small levels (fewer than kSmallLevelTiles tiles) are the coarsest ones;
 // their blocks come first in block index order (level 4 -> 0), so they are
 // the prefix [0, blocks) of the blocks.
@@ -235,8 +241,7 @@ void small_level_split(const Geometry &g, int &level_out, int &blocks)
 	level_out = kLevels;
 	for (int level = kLevels - 1; level >= 0; level--)
 	{
-		const int tiles = g.level[level].tiles_x * g.level[level].tiles_y * ((level == 0 && !g.chroma444) ? 1 : 3);
-		if (tiles >= kSmallLevelTiles)
+		if (level_tiles(g, level) >= kSmallLevelTiles)
 			break;
 		level_out = level;
 	}
@@ -1369,7 +1374,15 @@ struct pyrowave_decoder_opaque
 		return ok ? PYROWAVE_SUCCESS : PYROWAVE_ERROR_OUT_OF_DEVICE_MEMORY;
 	}
 
-	// Dequantise + inverse transform (pyrowave_decoder.cpp:796-830).
+	// Whether inverse level `level` shares a launch with the next finer one: both
+	// small (stripes), and the finer one has every component. With stage timing
+	// every level is a launch of its own.
+	bool pairs(int level) const
+	{
+		return !device->stage_timing && level % 2 == 0 && level >= 2 && level_tiles(g, level) < kSmallLevelTiles &&
+		       level_tiles(g, level - 1) < kSmallLevelTiles;
+	}
+
 	// Dequantise + inverse transform (pyrowave_decoder.cpp:796-830), as one graph launch.
 	bool run(const DecodeInput &in_args, const PlaneOutput &out, cudaStream_t s, bool dequant)
 	{
@@ -1401,7 +1414,14 @@ struct pyrowave_decoder_opaque
 			static const char *const idwt_tags[kLevels] = {"idwt0", "idwt1", "idwt2", "idwt3", "idwt4"};
 			for (int level = kLevels - 1; level >= 0; level--)
 			{
-				launch_idwt_level(lp[level], in, out, &band_maps[level], pdl && (dequant || level < kLevels - 1), s);
+				const bool programmatic = pdl && (dequant || level < kLevels - 1);
+				if (pairs(level))
+				{
+					level--;
+					launch_idwt_pair(lp[level], lp[level + 1], in, out, programmatic, s);
+				}
+				else
+					launch_idwt_level(lp[level], in, out, &band_maps[level], programmatic, s);
 				ok = ok && last_captured_node(s, dequant ? node_idwt_full[level] : node_idwt_only[level]);
 				timing.mark(device, s, idwt_tags[level]);
 			}
@@ -1422,9 +1442,14 @@ struct pyrowave_decoder_opaque
 			{
 				ok = set_kernel_args(graph.exec, node_dequant, bp, din);
 			}
-			for (int level = 0; level < kLevels; level++)
-				ok = ok && set_kernel_args(graph.exec, dequant ? node_idwt_full[level] : node_idwt_only[level], lp[level],
-				                           din, pout, band_maps[level]);
+			for (int level = kLevels - 1; level >= 0 && ok; level--)
+			{
+				const bool pair = pairs(level);
+				level -= pair ? 1 : 0;
+				const KernelNode &node = dequant ? node_idwt_full[level] : node_idwt_only[level];
+				ok = pair ? set_kernel_args(graph.exec, node, lp[level], lp[level + 1], din, pout)
+				          : set_kernel_args(graph.exec, node, lp[level], din, pout, band_maps[level]);
+			}
 			if (!ok)
 			{
 				graph.destroy();

@@ -434,6 +434,10 @@ void launch_dequant(const BlockParams &p, const DecodeInput &in, bool programmat
 void launch_idwt_level(const LevelParams &p, const DecodeInput &in, const PlaneOutput &out, const LevelTileMap *maps,
                        bool programmatic,
                        cudaStream_t stream);
+// Inverse levels p.level + 1 (`coarser`) and p.level in one launch; both small,
+// with the same components.
+void launch_idwt_pair(const LevelParams &p, const LevelParams &coarser, const DecodeInput &in, const PlaneOutput &out,
+                      bool programmatic, cudaStream_t stream);
 void launch_pyramid_io(const BlockParams &p, float *canonical, float *coef32, __half *coef16, bool to_canonical,
                        cudaStream_t stream);
 
