@@ -159,6 +159,23 @@ __device__ __forceinline__ void quant_analyze_row(const float *tile, const int l
 	max_wave = fminf(__fmul_rn(max_wave, qs), kMaxScaledMagnitude);
 	const int msb = float_msb(max_wave);
 	const int warp_msb = __reduce_max_sync(full, msb);
+	uint32_t *const code_word = buf.code_words + B.block8_offset + y8 * B.block8_stride + x8;
+	if (warp_msb < 0)
+	{
+		// Every value of the row quantises to zero: the packer does not look at its magnitudes.
+		if (r == 0)
+		{
+			if (lane < 16)
+			{
+				sh.dist[ly][lane] = 0.0f;
+				sh.cost[ly][lane] = 0u;
+			}
+			if (in_range && sub == 0)
+				*code_word = 0u;
+		}
+		return;
+	}
+
 	// Magnitudes as pairs (i, i + 4): the two lanes of a pair accumulate the two
 	// halves of the squared error, over i = 0..3 and i = 4..7, in the same order
 	// as eight scalar steps would.
@@ -196,23 +213,6 @@ __device__ __forceinline__ void quant_analyze_row(const float *tile, const int l
 		*reinterpret_cast<uint4 *>(buf.mag16 + int64_t(blk) * 1024 + 8 * (lane + 32 * ly)) =
 		    make_uint4(w[0], w[1], w[2], w[3]);
 	}
-	uint32_t *const code_word = buf.code_words + B.block8_offset + y8 * B.block8_stride + x8;
-	if (warp_msb < 0)
-	{
-		// Every value of the row quantises to zero.
-		if (r == 0)
-		{
-			if (lane < 16)
-			{
-				sh.dist[ly][lane] = 0.0f;
-				sh.cost[ly][lane] = 0u;
-			}
-			if (in_range && sub == 0)
-				*code_word = 0u;
-		}
-		return;
-	}
-
 	const float rdo = B.rdo_scale;
 
 	// Stats at q = 0 (wavelet_quant.comp:139-165,205-238): the 8x8's plane codes
@@ -1669,6 +1669,7 @@ __device__ __forceinline__ uint32_t compress_bytes(uint32_t x, uint32_t m)
 	return x;
 }
 
+constexpr int kPackEarlyBlocks = 148 * 32; // about what 56 registers let reside
 __device__ __forceinline__ void pack_body(uint32_t *const pkt, const BlockParams &p, const EncodeBuffers &buf, const int blk)
 {
 	const unsigned full = 0xffffffffu;
@@ -1683,6 +1684,11 @@ __device__ __forceinline__ void pack_body(uint32_t *const pkt, const BlockParams
 	// The resolve kernel releases this grid only after every quantiser has
 	// finished, so the quantised magnitudes and code words can be fetched before
 	// the wait; only the rate-control decisions come from the resolve kernel itself.
+	// That pays for frames whose blocks are all resident at once (kPackEarlyBlocks);
+	// beyond, half the blocks of a frame code nothing, and only the rows that do are
+	// read, once known.
+	const bool early = p.block_count_32x32 <= kPackEarlyBlocks;
+	const uint4 *const mags = reinterpret_cast<const uint4 *>(buf.mag16 + int64_t(blk) * 1024) + lane;
 	uint32_t cw[4];
 	uint4 sm[4];
 #pragma unroll
@@ -1691,7 +1697,7 @@ __device__ __forceinline__ void pack_body(uint32_t *const pkt, const BlockParams
 		const int y8 = by32 * 4 + h;
 		const bool in_range = x8 < L.blocks8_x && y8 < L.blocks8_y;
 		cw[h] = in_range ? __ldcg(&buf.code_words[B.block8_offset + y8 * B.block8_stride + x8]) : 0u;
-		sm[h] = __ldcg(reinterpret_cast<const uint4 *>(buf.mag16 + int64_t(blk) * 1024 + 8 * (lane + 32 * h)));
+		sm[h] = early ? __ldcg(mags + 32 * h) : make_uint4(0u, 0u, 0u, 0u);
 	}
 	pdl_wait();
 
@@ -1708,7 +1714,6 @@ __device__ __forceinline__ void pack_body(uint32_t *const pkt, const BlockParams
 	// the coded 8x8s and their plane bytes, in fields of packed words.
 	uint32_t ballot = 0, planes4 = 0, sig4 = 0, neg4 = 0;
 	uint32_t bytes01 = 0, bytes23 = 0;
-	const uint32_t threshold = (0x8000u - (1u << quant)) * 0x10001u;
 #pragma unroll
 	for (int h = 0; h < 4; h++)
 	{
@@ -1724,6 +1729,14 @@ __device__ __forceinline__ void pack_body(uint32_t *const pkt, const BlockParams
 			bytes01 |= nbytes << (16 * h);
 		else
 			bytes23 |= nbytes << (16 * (h - 2));
+		if (!early && wb != 0)
+			sm[h] = __ldcg(mags + 32 * h);
+	}
+	const uint32_t threshold = (0x8000u - (1u << quant)) * 0x10001u;
+#pragma unroll
+	for (int h = 0; h < 4; h++)
+	{
+		const uint32_t pl = (planes4 >> (8 * h)) & 0xffu;
 		// |int(v)| >> quant != 0, as a carry into the sign bit of each field.
 		const uint32_t w[4] = {sm[h].x, sm[h].y, sm[h].z, sm[h].w};
 		uint32_t ge[4];
