@@ -518,36 +518,21 @@ __device__ __forceinline__ void wait_finer_tiles(const int *xidx, const int *yid
 
 // Quantises the transmitted bands of a transformed tile in shared memory.
 template <int kThreads>
-__device__ __forceinline__ void quant_tile(DwtShared &sh, const LevelParams &p, const EncodeBuffers &buf, const int fused,
-                                           const int level, const int comp, const int tx, const int ty)
+__device__ __forceinline__ void quant_tile(DwtShared &sh, const LevelParams &p, const EncodeBuffers &buf, const int level,
+                                           const int comp, const int tx, const int ty)
 {
 	using Split = DwtSplit<kThreads, 1>;
 	const LevelDesc &L = p.L;
 	// Quantise the transmitted bands of this tile: HL, LH, HH (+ LL at the last
-	// level), kGroups bands per round. With fused == kFusedSplitTail, a last
-	// round that would leave groups idle (HH after HL and LH in a 256-thread
-	// CTA) instead runs its band on the whole CTA with twice the threads per
-	// sub-block: same results, a shorter serial chain for levels of few waves.
+	// level), kGroups bands per round. (A last round on the whole CTA, two warps
+	// per row, repeats the rows' fixed work: 1080p encode 42.25 against 41.4 us.)
 	const int first_band = level == kLevels - 1 ? 0 : 1;
 	const int nb = 4 - first_band;
 	const int grp = threadIdx.x / Split::kGroupThreads, t = threadIdx.x % Split::kGroupThreads;
 	const int ly = (t >> 5) & 3;
-	bool split_tail = false;
-	if constexpr (kThreads == kLargeLevelThreads)
-		split_tail = fused == kFusedSplitTail && (nb % Split::kGroups) != 0;
-	const int rounds = split_tail ? nb / Split::kGroups : (nb + Split::kGroups - 1) / Split::kGroups;
-	for (int bi = grp; bi < min(nb, rounds * Split::kGroups); bi += Split::kGroups)
+	for (int bi = grp; bi < nb; bi += Split::kGroups)
 		quant_analyze_row<Split::kQSplit>(&sh.bands[first_band + bi][0][0], ly, t >> 7, sh.q[bi], sh.scales[bi], L,
 		                                  p.band[comp][first_band + bi], tx, ty, buf);
-	if constexpr (kThreads == kLargeLevelThreads)
-	{
-		if (split_tail)
-		{
-			const int bi = rounds * Split::kGroups;
-			quant_analyze_row<2 * Split::kQSplit>(&sh.bands[first_band + bi][0][0], ly, int(threadIdx.x) >> 7, sh.q[bi],
-			                                      sh.scales[bi], L, p.band[comp][first_band + bi], tx, ty, buf);
-		}
-	}
 	__syncthreads();
 	// A half-warp per band finishes its block. Tile dataflow: the resolve waits for
 	// the count of every CTA, released once after all of its bands' rows (a full
@@ -965,7 +950,7 @@ __device__ __forceinline__ void dwt_forward_body(DwtSharedT<DwtSplit<kThreads, k
 			return;
 		if (!buf.tile_done)
 			__syncthreads();
-		quant_tile<kThreads>(sh, p, buf, fused, level, comp, tx, ty);
+		quant_tile<kThreads>(sh, p, buf, level, comp, tx, ty);
 	}
 }
 
@@ -2143,19 +2128,11 @@ LaunchConfig::LaunchConfig(dim3 grid, dim3 block, cudaStream_t stream, bool prog
 	cfg.numAttrs = programmatic ? 1 : 0;
 }
 
-int forward_fused_mode(const LevelParams &p, bool fused_quant)
-{
-	if (!fused_quant)
-		return 0;
-	const int tiles = p.L.tiles_x * p.L.tiles_y * ((p.level == 0 && !p.chroma444) ? 1 : 3);
-	return tiles < kSplitTailTiles ? kFusedSplitTail : 1;
-}
-
 void launch_dwt_forward_level(const LevelParams &p, const PlaneInput &in, const EncodeBuffers &buf,
                               bool fused_quant, bool programmatic, cudaStream_t stream)
 {
 	const dim3 grid(p.L.tiles_x * p.L.tiles_y, (p.level == 0 && !p.chroma444) ? 1 : 3);
-	const int f = forward_fused_mode(p, fused_quant);
+	const int f = fused_quant ? 1 : 0;
 	const bool half = p.L.fp16 || p.L.stage16 || (p.level > 0 && p.P.fp16);
 	if (int(grid.x * grid.y) < kSmallLevelTiles && f == 0)
 	{

@@ -984,7 +984,7 @@ struct pyrowave_encoder_opaque
 			bool ok = true;
 			for (int level = 0; level < kLevels; level++)
 			{
-				int fused = forward_fused_mode(lp[level], level < small_level);
+				int fused = level < small_level ? 1 : 0;
 				ok = ok && set_kernel_args(graph.exec, node_dwt[level], lp[level], pin, b, fused);
 			}
 			ok = ok && set_kernel_args(graph.exec, node_resolve, rp, b);

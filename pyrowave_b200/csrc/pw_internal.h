@@ -406,19 +406,12 @@ void launch_batch_persistent(const BatchRunParams &rp, int ctas, cudaStream_t st
 // launch across the whole GPU after the last level instead of inside the
 // transform of each level.
 constexpr int kSmallLevelTiles = 256;
-// Fused quantiser modes of a forward level launch: 0 none, 1 fused, and
-// kFusedSplitTail (levels of fewer than kSplitTailTiles tiles, about two waves
-// of 256-thread CTAs): a last quantiser round with idle groups runs on the
-// whole CTA instead.
-constexpr int kFusedSplitTail = 2;
-constexpr int kSplitTailTiles = 2 * 148 * 4;
 // CTAs per tile of a small transform-only level (row stripes of the tile).
 constexpr int kDwtStripeCtas = 4;
 // Bounded waits of the tile dataflow (each poll sleeps about 64 ns or more):
 // about a second at most, after which the waiting CTA records kErrorLevelWait
 // and carries on.
 constexpr uint32_t kDataflowWaitSpins = 1u << 20;
-int forward_fused_mode(const LevelParams &p, bool fused_quant);
 void launch_dwt_forward_level(const LevelParams &p, const PlaneInput &in, const EncodeBuffers &buf,
                               bool fused_quant, bool programmatic, cudaStream_t stream);
 // Quantise and analyse the first nblocks 32x32 blocks (block index order) from storage.
