@@ -1106,8 +1106,9 @@ __global__ void __launch_bounds__(256 * S) quant_blocks_batch_kernel(const Batch
 
 // ---------------------------------------------------------------------------
 // Block-wide exclusive scan (blockDim.x a multiple of 32, at most 1024);
-// returns the exclusive prefix and the block total.
-template <typename T> __device__ __forceinline__ T block_exclusive_scan(T v, T *warp_sums, T &total)
+// returns the exclusive prefix and the block total. With kReuse it ends with a
+// barrier, after which warp_sums may be used again.
+template <bool kReuse = true, typename T> __device__ __forceinline__ T block_exclusive_scan(T v, T *warp_sums, T &total)
 {
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
 	T x = v;
@@ -1136,7 +1137,8 @@ template <typename T> __device__ __forceinline__ T block_exclusive_scan(T v, T *
 	__syncthreads();
 	const T base = warp == 0 ? T(0) : warp_sums[warp - 1];
 	total = warp_sums[nwarps - 1];
-	__syncthreads();
+	if (kReuse)
+		__syncthreads();
 	return base + x - v;
 }
 
@@ -1454,10 +1456,10 @@ template <int R>
 __global__ void __launch_bounds__(kClusterResolveThreads, 1)
     resolve_cluster_kernel(const ResolveParams p, const EncodeBuffers buf)
 {
-	__shared__ uint32_t scan[kHistSize];
-	__shared__ uint32_t warp_sums[32];
+	__shared__ uint32_t warp_sums[2][32]; // one per scan: no barrier to reuse it
 	__shared__ unsigned long long warp_sums64[32];
 	__shared__ int s_xstar;
+	__shared__ uint32_t s_before; // savings of the slots before x*
 	__shared__ unsigned long long s_saving_totals[kMaxResolveCluster]; // [r]: savings total of rank r < this rank
 	__shared__ unsigned long long s_word_totals[kMaxResolveCluster];   // [r]: words << 32 | non-empty << 1 of rank r
 	// Peers write into this CTA's shared memory only after every CTA started.
@@ -1482,18 +1484,23 @@ __global__ void __launch_bounds__(kClusterResolveThreads, 1)
 	if (t == 0)
 		s_xstar = -1;
 	uint32_t total;
-	const uint32_t run = block_exclusive_scan(h0 + h1, warp_sums, total);
-	scan[2 * t] = run + h0;
-	scan[2 * t + 1] = run + h0 + h1;
-	__syncthreads();
+	const uint32_t run = block_exclusive_scan<false>(h0 + h1, warp_sums[0], total);
 
 	// No block codes words at quant 15, so a block's savings add up to its words at quant 0.
 	const int64_t need = int64_t(total) - int64_t(p.target_words);
 	if (need > 0)
 	{
-		for (int x = 2 * t; x < 2 * t + 2; x++)
-			if (int64_t(scan[x]) >= need && (x == 0 || int64_t(scan[x - 1]) < need))
-				s_xstar = x;
+		// The first slot whose inclusive prefix reaches the need (exactly one slot's does first).
+		if (int64_t(run + h0) >= need && (t == 0 || int64_t(run) < need))
+		{
+			s_xstar = 2 * t;
+			s_before = run;
+		}
+		if (int64_t(run + h0 + h1) >= need && int64_t(run + h0) < need)
+		{
+			s_xstar = 2 * t + 1;
+			s_before = run + h0;
+		}
 	}
 	__syncthreads();
 	const int xstar = s_xstar; // the same in every CTA: each scanned the same histogram
@@ -1508,7 +1515,7 @@ __global__ void __launch_bounds__(kClusterResolveThreads, 1)
 	{
 		const int start = (xstar & (kSubdivisions - 1)) * p.blocks_per_subdivision;
 		const int end = min(start + p.blocks_per_subdivision, n);
-		const int64_t required = need - (xstar > 0 ? int64_t(scan[xstar - 1]) : 0);
+		const int64_t required = need - int64_t(s_before);
 		const uint32_t bk = uint32_t(xstar >> 4);
 		uint32_t sv[R];
 		uint32_t local = 0;
@@ -1520,7 +1527,7 @@ __global__ void __launch_bounds__(kClusterResolveThreads, 1)
 			local += sv[i];
 		}
 		uint32_t cta_total;
-		uint32_t ex = block_exclusive_scan(local, warp_sums, cta_total);
+		uint32_t ex = block_exclusive_scan<false>(local, warp_sums[1], cta_total);
 		// When the x* subdivision lies inside one CTA's blocks (every CTA sees
 		// the same x*, so all take the same branch), the other CTAs hold none of
 		// its savings and the prefix needs no exchange.
@@ -1560,7 +1567,7 @@ __global__ void __launch_bounds__(kClusterResolveThreads, 1)
 		}
 	}
 	unsigned long long cta_words;
-	unsigned long long pos = block_exclusive_scan(local, warp_sums64, cta_words);
+	unsigned long long pos = block_exclusive_scan<false>(local, warp_sums64, cta_words);
 	if (t < int(ncta) && t > int(rank))
 		st_cluster_u64(&s_word_totals[rank], uint32_t(t), cta_words);
 	cluster_sync();
