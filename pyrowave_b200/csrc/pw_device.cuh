@@ -148,6 +148,14 @@ __device__ __forceinline__ void red_release_add(uint32_t *c, uint32_t v)
 	asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(c), "r"(v) : "memory");
 }
 
+// Adds to a counter and returns its value before, ordered both ways for the calling thread.
+__device__ __forceinline__ uint32_t atom_acq_rel_add(uint32_t *c, uint32_t v)
+{
+	uint32_t old;
+	asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(c), "r"(v) : "memory");
+	return old;
+}
+
 // Adds one to a counter once every thread of the CTA has stored its part
 // (called by every thread; the barrier orders the CTA's stores before the
 // release of one thread of the last warp, which has the least left to do).

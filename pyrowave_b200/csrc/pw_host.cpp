@@ -1116,7 +1116,7 @@ struct pyrowave_decoder_opaque
 	uint32_t *pk_summaries = nullptr;
 	size_t pk_capacity = 0; // packets
 	uint32_t *pk_items = nullptr;
-	size_t pk_items_capacity = 0; // words
+	size_t pk_items_capacity = 0; // words of each half (positions, blocks)
 	unsigned long long *pk_first = nullptr;
 	PacketStatus *pk_status = nullptr;
 	PacketStatus *pk_status_h = nullptr;
@@ -1514,7 +1514,7 @@ struct pyrowave_decoder_opaque
 			cudaStreamSynchronize(s);
 			dev_free(pk_items);
 			const size_t cap = std::max<size_t>(data_words, 1 << 16);
-			pk_items = dev_alloc<uint32_t>(cap, ok);
+			pk_items = dev_alloc<uint32_t>(2 * cap, ok);
 			pk_items_capacity = ok ? cap : 0;
 		}
 		if (!ok)
@@ -1532,6 +1532,7 @@ struct pyrowave_decoder_opaque
 		pp.state_before = pk_state;
 		pp.summaries = pk_summaries;
 		pp.items = pk_items;
+		pp.item_blocks = pk_items + pk_items_capacity;
 		pp.first = pk_first;
 		pp.counter = pk_counter;
 		pp.status = pk_status;

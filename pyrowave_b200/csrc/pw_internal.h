@@ -457,6 +457,7 @@ struct PacketParams
 	uint8_t *state_before;            // count
 	uint32_t *summaries;              // count x 8 words: each packet's item summary
 	uint32_t *items;                  // data_bytes / 4: packet p's item positions at its own first word on
+	uint32_t *item_blocks;            // likewise the items' block indices, ~0 for a sequence header
 	unsigned long long *first;        // block_count: smallest (packet, item, word offset) key, ~0 = missing
 	uint32_t *counter;                // CTAs of the table pass done (zero between calls)
 	PacketStatus *status;

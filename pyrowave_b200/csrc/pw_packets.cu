@@ -13,8 +13,8 @@
 //      it, the block total of the last accepted sequence header, and whether
 //      the parser rejects it. The last CTA to finish scans the state maps of
 //      all packets: the state before each packet, the last restart of the
-//      whole list, the frame's sequence and block total; it also clears the
-//      first-copy table.
+//      whole list, the frame's sequence and block total. Meanwhile every CTA
+//      clears its share of the first-copy table.
 //   2. packet_blocks_kernel  one CTA per packet from the last restart on:
 //      every block the parser keeps proposes (packet, item, word offset) and
 //      the smallest, the first copy pushed, wins by a 64-bit atomicMin; the
@@ -30,6 +30,7 @@ constexpr uint32_t kNoPos = 0xffffu;        // no restart inside the packet
 constexpr uint32_t kNoTotal = 0xffffffffu;  // no sequence header accepted
 constexpr uint32_t kMaxItems = 1u << 14;    // items (headers + blocks) per packet
 constexpr unsigned long long kNoKey = ~0ull;
+constexpr uint32_t kNoBlock = 0xffffffffu;  // listed item is a sequence header
 
 struct WalkResult
 {
@@ -132,27 +133,30 @@ __device__ __forceinline__ bool packet_span(const PacketParams &pp, int p, uint3
 // Every word position p gets next(p) in parallel: the position after an item
 // starting at p, or where the parser stops (an item it rejects, the end, fewer
 // than 8 bytes left). Three doubling passes give next^8; one thread follows it
-// from 0 (one shared-memory load per 8 items), the items between those anchors
-// are filled in parallel, and every later step runs over the items in
-// parallel. Packets whose items share one sequence number (every packet of a
-// frame) need no walk at all: the parser's state change has a closed form.
-// Other packets are walked item by item.
+// from 0 (one shared-memory load per 8 items), and one thread per anchor lists
+// and summarises the items up to the next one. Packets whose items share one
+// sequence number (every packet of a frame) need no walk at all: the parser's
+// state change has a closed form. Other packets are walked item by item.
+//
+// Bound by latency: a chain of memory round trips, barriers of the CTA and the
+// chase, with one CTA per packet. So words are classified straight from the
+// loads, the summary is taken while listing, and 16-bit positions leave room
+// for two CTAs per SM.
 constexpr int kFastWords = 8192;  // packets up to 32 KiB take this path
-constexpr uint32_t kDone = 0xffffffffu; // the item ends the packet exactly
-constexpr uint32_t kStop = 0xfffffffeu; // the parser rejects the item
-constexpr uint32_t kLeft = 0xfffffffdu; // fewer than 8 bytes left: not an item
+// Codes of next(p) that are not positions.
+constexpr uint32_t kLeft = 0xfffdu; // fewer than 8 bytes left: not an item
+constexpr uint32_t kStop = 0xfffeu; // the parser rejects the item
+constexpr uint32_t kDone = 0xffffu; // the item ends the packet exactly
 constexpr int kPacketThreads = 1024;
-constexpr uint16_t kJumpEnd = 0xffffu;
-constexpr int kAnchorRounds = 3;                 // the chase follows next^8
+constexpr int kAnchorRounds = 3; // the chase follows next^8
 constexpr int kAnchorStep = 1 << kAnchorRounds;
 
 struct PacketSmem
 {
 	uint32_t words[kFastWords];
-	uint32_t next[kFastWords];
-	uint32_t items[kFastWords / 2 + 2]; // item start positions in push order
-	uint16_t jump[2][kFastWords];        // next^(2^r), kJumpEnd where the chain stops first
-	uint16_t anchors[kFastWords / 16 + 2]; // every kAnchorStep-th item
+	uint16_t next[kFastWords];
+	uint16_t jump[2][kFastWords];                   // next^(2^r), a code (>= kLeft) where the chain stops first
+	uint16_t anchors[kFastWords / (2 * kAnchorStep) + 2]; // every kAnchorStep-th item
 };
 constexpr size_t kPacketSmemBytes = sizeof(PacketSmem);
 
@@ -175,10 +179,9 @@ struct ItemInfo
 	uint32_t error; // 0, 1 (before the sequence check), 2 (after it)
 };
 
-__device__ __forceinline__ ItemInfo classify(const uint32_t *w, uint32_t p, uint32_t rem, const PacketParams &pp)
+__device__ __forceinline__ ItemInfo classify(uint32_t w0, uint32_t w1, uint32_t rem, const PacketParams &pp)
 {
 	ItemInfo it;
-	const uint32_t w0 = w[p], w1 = w[p + 1];
 	it.header = (w0 >> 31) & 1u;
 	it.seq = (w0 >> 28) & 7u;
 	it.total = w1 & 0xffffffu;
@@ -203,28 +206,38 @@ __device__ __forceinline__ ItemInfo classify(const uint32_t *w, uint32_t p, uint
 	return it;
 }
 
-// Stages the packet (nwords <= kFastWords), lists its items in sm.items and
-// fills the item summary. Every thread of the CTA calls it.
+// Stages the packet (nwords <= kFastWords), lists its items in pp.items and
+// pp.item_blocks and fills the item summary. Every thread of the CTA calls it.
 __device__ void discover_items(PacketSmem &sm, ItemSummary &sum, const PacketParams &pp, uint32_t first,
                                uint32_t size, uint32_t nwords)
 {
 	const int t = threadIdx.x;
-	// Stage: eight loads in flight per thread.
-	for (uint32_t base = 0; base < nwords; base += 8 * kPacketThreads)
+	constexpr int kLoads = 4; // words in flight per thread, each with its successor
+	for (uint32_t base = t; base < nwords; base += kLoads * kPacketThreads)
 	{
-		uint32_t v[8];
+		uint32_t w0[kLoads], w1[kLoads];
 #pragma unroll
-		for (int u = 0; u < 8; u++)
+		for (int u = 0; u < kLoads; u++)
 		{
-			const uint32_t i = base + t + u * kPacketThreads;
-			v[u] = i < nwords ? __ldg(pp.data + first + i) : 0u;
+			const uint32_t p = base + u * kPacketThreads;
+			w0[u] = p < nwords ? __ldg(pp.data + first + p) : 0u;
+			w1[u] = p + 1 < nwords ? __ldg(pp.data + first + p + 1) : 0u;
 		}
 #pragma unroll
-		for (int u = 0; u < 8; u++)
+		for (int u = 0; u < kLoads; u++)
 		{
-			const uint32_t i = base + t + u * kPacketThreads;
-			if (i < nwords)
-				sm.words[i] = v[u];
+			const uint32_t p = base + u * kPacketThreads;
+			if (p >= nwords)
+				break;
+			sm.words[p] = w0[u];
+			const uint32_t rem = size - 4 * p;
+			uint32_t nxt = kLeft;
+			if (rem >= 8)
+			{
+				const ItemInfo it = classify(w0[u], w1[u], rem, pp);
+				nxt = it.error ? kStop : (p + it.words < nwords ? p + it.words : kDone);
+			}
+			sm.next[p] = uint16_t(nxt);
 		}
 	}
 	if (t == 0)
@@ -237,36 +250,18 @@ __device__ void discover_items(PacketSmem &sm, ItemSummary &sum, const PacketPar
 		sum.last_header = 0;
 	}
 	__syncthreads();
-	for (uint32_t p = t; p < nwords; p += kPacketThreads)
-	{
-		const uint32_t rem = size - 4 * p;
-		uint32_t nxt = kLeft;
-		if (rem >= 8)
-		{
-			const ItemInfo it = classify(sm.words, p, rem, pp);
-			nxt = it.error ? kStop : (p + it.words < nwords ? p + it.words : kDone);
-		}
-		sm.next[p] = nxt;
-	}
-	__syncthreads();
-	// next^8 by three doubling passes; one thread then follows it from 0 (one
-	// load per 8 items) and the items between anchors are filled in parallel.
-	for (uint32_t p = t; p < nwords; p += kPacketThreads)
-	{
-		const uint32_t nx = sm.next[p];
-		sm.jump[0][p] = nx < nwords ? uint16_t(nx) : kJumpEnd;
-	}
-	__syncthreads();
-	int cur = 0;
+	const uint16_t *src = sm.next;
+#pragma unroll
 	for (int r = 0; r < kAnchorRounds; r++)
 	{
+		uint16_t *const dst = sm.jump[r & 1];
 		for (uint32_t p = t; p < nwords; p += kPacketThreads)
 		{
-			const uint32_t j = sm.jump[cur][p];
-			sm.jump[cur ^ 1][p] = j == kJumpEnd ? kJumpEnd : sm.jump[cur][j];
+			const uint32_t j = src[p];
+			dst[p] = j >= kLeft ? uint16_t(j) : src[j];
 		}
 		__syncthreads();
-		cur ^= 1;
+		src = dst;
 	}
 	__shared__ uint32_t s_anchors;
 	if (t == 0)
@@ -275,70 +270,59 @@ __device__ void discover_items(PacketSmem &sm, ItemSummary &sum, const PacketPar
 		while (nwords > 0)
 		{
 			sm.anchors[m++] = uint16_t(p);
-			const uint32_t j = sm.jump[cur][p];
-			if (j == kJumpEnd)
+			p = src[p];
+			if (p >= kLeft)
 				break;
-			p = j;
 		}
 		s_anchors = m;
 	}
 	__syncthreads();
 	const uint32_t na = s_anchors;
+	// The sequence range covers the items whose sequence number the parser
+	// looks at. Only the last item can be rejected.
+	uint32_t smin = 7, smax = 0;
 	for (uint32_t a = t; a < na; a += kPacketThreads)
 	{
 		uint32_t q = sm.anchors[a];
 		for (uint32_t i = 0; i < uint32_t(kAnchorStep); i++)
 		{
-			const uint32_t nx = sm.next[q];
+			const uint32_t k = a * kAnchorStep + i, nx = sm.next[q];
 			if (nx == kLeft)
 			{
 				sum.trailing = 1; // q is not an item: fewer than 8 bytes were left
-				sum.nitems = a * kAnchorStep + i;
+				sum.nitems = k;
 				break;
 			}
-			sm.items[a * kAnchorStep + i] = q;
-			if (nx == kStop || nx == kDone)
+			const ItemInfo it = classify(sm.words[q], sm.words[q + 1], size - 4 * q, pp);
+			pp.items[first + k] = q;
+			pp.item_blocks[first + k] = it.header ? kNoBlock : it.block;
+			if (it.error)
+				sum.error = k << 2 | it.error;
+			else if (it.header)
+				atomicMax(&sum.last_header, (unsigned long long)(k + 1) << 32 | it.total);
+			if (it.error != 1)
 			{
-				sum.nitems = a * kAnchorStep + i + 1;
+				smin = min(smin, it.seq);
+				smax = max(smax, it.seq);
+			}
+			if (nx >= kLeft)
+			{
+				sum.nitems = k + 1;
 				break;
 			}
 			q = nx;
 		}
 	}
-	__syncthreads();
-	const uint32_t n = sum.nitems;
-	for (uint32_t k = t; k < n; k += kPacketThreads)
+	if (uint32_t(t & ~31) < na) // uniform over the warp
 	{
-		const uint32_t p = sm.items[k];
-		const ItemInfo it = classify(sm.words, p, size - 4 * p, pp);
-		if (it.error)
-			atomicMin(&sum.error, k << 2 | it.error); // only the last item can be rejected
+		smin = __reduce_min_sync(0xffffffffu, smin);
+		smax = __reduce_max_sync(0xffffffffu, smax);
+		if ((t & 31) == 0 && smin <= smax)
+		{
+			atomicMin(&sum.seq_min, smin);
+			atomicMax(&sum.seq_max, smax);
+		}
 	}
-	__syncthreads();
-	// Sequence range of the items whose sequence number the parser looks at,
-	// and the last accepted header.
-	const uint32_t err_item = sum.error == ~0u ? ~0u : sum.error >> 2;
-	const uint32_t err_kind = sum.error == ~0u ? 0u : sum.error & 3u;
-	uint32_t smin = 7, smax = 0;
-	unsigned long long lh = 0;
-	for (uint32_t k = t; k < n; k += kPacketThreads)
-	{
-		if (k == err_item && err_kind == 1)
-			continue;
-		const uint32_t p = sm.items[k];
-		const ItemInfo it = classify(sm.words, p, size - 4 * p, pp);
-		smin = min(smin, it.seq);
-		smax = max(smax, it.seq);
-		if (it.header && k != err_item)
-			lh = max(lh, (unsigned long long)(k + 1) << 32 | it.total);
-	}
-	if (smin <= smax)
-	{
-		atomicMin(&sum.seq_min, smin);
-		atomicMax(&sum.seq_max, smax);
-	}
-	if (lh)
-		atomicMax(&sum.last_header, lh);
 	__syncthreads();
 }
 
@@ -423,6 +407,7 @@ __device__ void scan_packets(const PacketParams &pp)
 	// warp by shuffles, then over the warp totals. Warps past the last packet
 	// hold the identity.
 	const bool active = warp * 32 * per < n; // uniform over the warp
+	const int warps = (n + 32 * per - 1) / (32 * per);
 	unsigned long long incl = kIdentityMap;
 	for (int p = p0; p < p1; p++)
 		incl = compose(incl, packet_map(pp, p));
@@ -442,14 +427,13 @@ __device__ void scan_packets(const PacketParams &pp)
 	if (warp == 0)
 	{
 		unsigned long long w = s_warp[lane];
-#pragma unroll
-		for (int off = 1; off < 32; off *= 2)
+		for (int off = 1; off < warps; off *= 2)
 		{
 			const unsigned long long other = __shfl_up_sync(0xffffffffu, w, off);
 			if (lane >= off)
 				w = compose(other, w);
 		}
-		s_warp[lane] = w; // inclusive over warps
+		s_warp[lane] = w; // inclusive over the active warps
 	}
 	__syncthreads();
 	unsigned long long excl = active ? __shfl_up_sync(0xffffffffu, incl, 1) : kIdentityMap;
@@ -481,13 +465,11 @@ __device__ void scan_packets(const PacketParams &pp)
 		atomicMax(&s_last_total, last_total);
 	if (invalid)
 		atomicAdd(&s_invalid, invalid);
-	for (int b = t; b < pp.block_count; b += 1024)
-		pp.first[b] = kNoKey;
 	__syncthreads();
 	if (t == 0)
 	{
 		PacketStatus st = {};
-		const uint32_t final_state = n > 0 ? map_at(s_warp[31], kNoneState) : kNoneState;
+		const uint32_t final_state = n > 0 ? map_at(s_warp[warps - 1], kNoneState) : kNoneState;
 		st.sequence = final_state == kNoneState ? 0xffffffffu : final_state - 1;
 		st.invalid_packets = s_invalid;
 		const unsigned long long lr = s_last_restart;
@@ -515,13 +497,10 @@ __global__ void __launch_bounds__(kPacketThreads) packet_tables_kernel(const Pac
 	const uint32_t nwords = (size + 3) / 4;
 	const bool fast = ok && nwords <= uint32_t(kFastWords);
 	pdl_trigger(); // the block pass may launch meanwhile
+	for (int b = p * kPacketThreads + int(threadIdx.x); b < pp.block_count; b += pp.count * kPacketThreads)
+		pp.first[b] = kNoKey;
 	if (fast)
-	{
 		discover_items(sm, sum, pp, first, size, nwords);
-		// The item list goes to the packet's own word range of pp.items, for the block pass.
-		for (uint32_t k = threadIdx.x; k < sum.nitems; k += kPacketThreads)
-			pp.items[first + k] = sm.items[k];
-	}
 	if (threadIdx.x == 0)
 	{
 		ItemSummary rec = fast ? sum : ItemSummary{};
@@ -546,17 +525,19 @@ __global__ void __launch_bounds__(kPacketThreads) packet_tables_kernel(const Pac
 	pp.tables[(size_t(p) * 9 + init) * 2 + 0] = r.state | (r.error ? 16u : 0u) | (r.restart << 8);
 	pp.tables[(size_t(p) * 9 + init) * 2 + 1] = r.total;
 	}
-	// The last CTA to finish scans every packet's table (threadfence reduction:
-	// no CTA waits for another).
+	// The last CTA to finish scans every packet's table (no CTA waits for
+	// another). The tables are the first warp's stores, so its first thread's
+	// release covers them; the rest is for the next kernel.
 	__shared__ uint32_t s_ticket;
-	__threadfence();
-	__syncthreads();
-	if (threadIdx.x == 0)
-		s_ticket = atomicAdd(pp.counter, 1u);
+	if (threadIdx.x < 32)
+	{
+		__syncwarp();
+		if (threadIdx.x == 0)
+			s_ticket = atom_acq_rel_add(pp.counter, 1u);
+	}
 	__syncthreads();
 	if (s_ticket != uint32_t(pp.count) - 1)
 		return;
-	__threadfence();
 	if (threadIdx.x == 0)
 		*pp.counter = 0; // ready for the next call
 	scan_packets(pp);
@@ -570,22 +551,26 @@ __global__ void __launch_bounds__(256) packet_blocks_kernel(const PacketParams p
 	const bool ok = packet_span(pp, p, first, size);
 	const uint32_t nwords = (size + 3) / 4;
 	pdl_wait();
+	// One round trip: the state, the summary and the thread's first item (which
+	// need not exist, but its place does) are read before they are known to count.
 	const uint32_t rp = __ldcg(&pp.status->restart_packet), ri = __ldcg(&pp.status->restart_item);
 	const uint32_t seq = __ldcg(&pp.status->sequence);
-	if (!ok || seq == 0xffffffffu || uint32_t(p) < rp)
-		return; // uniform over the CTA
 	const uint32_t state = pp.state_before[p];
 	const ItemSummary sum = reinterpret_cast<const ItemSummary *>(pp.summaries)[p];
-	__shared__ uint32_t s_new;
-	if (threadIdx.x == 0)
-		s_new = 0;
-	__syncthreads();
+	uint32_t pos = 0, block = kNoBlock;
+	if (ok && threadIdx.x < nwords)
+	{
+		pos = __ldcg(pp.items + first + threadIdx.x);
+		block = __ldcg(pp.item_blocks + first + threadIdx.x);
+	}
+	if (!ok || seq == 0xffffffffu || uint32_t(p) < rp)
+		return; // uniform over the CTA
 	uint32_t fresh = 0; // blocks this thread saw first
-	auto keep = [&](uint32_t block, uint32_t pos, uint32_t item) {
+	auto keep = [&](uint32_t b, uint32_t word, uint32_t item) {
 		if (uint32_t(p) == rp && item < ri)
 			return; // before the last restart: cleared
-		const unsigned long long key = (unsigned long long)p << 44 | (unsigned long long)item << 30 | (first + pos);
-		if (atomicMin(pp.first + block, key) == kNoKey)
+		const unsigned long long key = (unsigned long long)p << 44 | (unsigned long long)item << 30 | (first + word);
+		if (atomicMin(pp.first + b, key) == kNoKey)
 			fresh++;
 	};
 	if (sum.fast && sum.seq_min == sum.seq_max)
@@ -596,23 +581,20 @@ __global__ void __launch_bounds__(256) packet_blocks_kernel(const PacketParams p
 		const uint32_t n = accepts ? min(sum.nitems, err_item) : 0u;
 		for (uint32_t k = threadIdx.x; k < n; k += blockDim.x)
 		{
-			const uint32_t q = __ldcg(pp.items + first + k);
-			if (q + 1 >= nwords)
-				continue;
-			const uint32_t w0 = __ldg(pp.data + first + q), w1 = __ldg(pp.data + first + q + 1);
-			const uint32_t block = (w1 >> 8) & 0xffffffu;
-			if (((w0 >> 31) & 1u) || block >= uint32_t(pp.block_count))
-				continue; // a sequence header
-			keep(block, q, k);
+			if (k >= blockDim.x)
+			{
+				pos = __ldcg(pp.items + first + k);
+				block = __ldcg(pp.item_blocks + first + k);
+			}
+			if (pos + 1 < nwords && block < uint32_t(pp.block_count)) // not a sequence header
+				keep(block, pos, k);
 		}
 	}
 	else if (threadIdx.x == 0)
 		walk_packet([&](uint32_t i) { return i < nwords ? __ldg(pp.data + first + i) : 0u; }, size, state, pp, keep);
-	if (fresh)
-		atomicAdd(&s_new, fresh);
-	__syncthreads();
-	if (threadIdx.x == 0 && s_new)
-		atomicAdd(&pp.status->decoded_blocks, s_new);
+	fresh = __reduce_add_sync(0xffffffffu, fresh);
+	if ((threadIdx.x & 31) == 0 && fresh)
+		atomicAdd(&pp.status->decoded_blocks, fresh);
 }
 
 } // namespace
