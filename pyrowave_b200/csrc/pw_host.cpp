@@ -1100,9 +1100,13 @@ struct pyrowave_decoder_opaque
 	uint32_t *h_upload = nullptr;
 	size_t h_upload_capacity = 0;
 	StageEvents timing;
-	CapturedGraph graph_full, graph_idwt;
-	KernelNode node_dequant;
-	KernelNode node_idwt_full[kLevels], node_idwt_only[kLevels];
+	// One decode sequence as a graph, and its kernel nodes.
+	struct DecodeGraph
+	{
+		CapturedGraph graph;
+		KernelNode packet_tables, packet_blocks, dequant, idwt[kLevels];
+	};
+	DecodeGraph graph_full, graph_idwt, graph_packets;
 
 	LevelTileMap band_maps[kLevels] = {}; // TMA maps of the FP32 bands (inverse transform tile loads)
 	DecodeState *state_d = nullptr;  // per-decode state: error bits
@@ -1278,8 +1282,9 @@ struct pyrowave_decoder_opaque
 		pk_capacity = 0;
 		pk_pending = false;
 		timing.destroy();
-		graph_full.destroy();
-		graph_idwt.destroy();
+		graph_full.graph.destroy();
+		graph_idwt.graph.destroy();
+		graph_packets.graph.destroy();
 		coef32 = nullptr;
 		coef16 = nullptr;
 		jobs_d = offsets_d = payload_d = nullptr;
@@ -1383,21 +1388,31 @@ struct pyrowave_decoder_opaque
 		       level_tiles(g, level - 1) < kSmallLevelTiles;
 	}
 
-	// Dequantise + inverse transform (pyrowave_decoder.cpp:796-830), as one graph launch.
-	bool run(const DecodeInput &in_args, const PlaneOutput &out, cudaStream_t s, bool dequant)
+	// Dequantise + inverse transform (pyrowave_decoder.cpp:796-830), as one graph launch,
+	// after the packet assembly where `packets` is given.
+	bool run(const DecodeInput &in_args, const PlaneOutput &out, cudaStream_t s, bool dequant,
+	         const PacketParams *packets = nullptr)
 	{
 		DecodeInput in = in_args;
 		in.error = error_d;
 		in.state = state_d;
 		timing.collect(device);
 		timing.prepare(device);
-		CapturedGraph &graph = dequant ? graph_full : graph_idwt;
+		DecodeGraph &nodes = packets ? graph_packets : dequant ? graph_full : graph_idwt;
+		CapturedGraph &graph = nodes.graph;
 		const uint64_t key = device->stage_timing ? 1ull : 0ull;
 		if (!graph.valid() || graph.key != key)
 		{
 			if (!graph.begin(s))
 				return false;
 			bool ok = true;
+			if (packets)
+			{
+				launch_packet_tables(*packets, s);
+				ok = ok && last_captured_node(s, nodes.packet_tables);
+				launch_packet_blocks(*packets, s);
+				ok = ok && last_captured_node(s, nodes.packet_blocks);
+			}
 			timing.begin(device, s);
 			const bool pdl = !device->stage_timing; // event nodes between kernels break programmatic edges
 			// The dequantiser clears the decode state before any inverse level runs;
@@ -1406,8 +1421,8 @@ struct pyrowave_decoder_opaque
 				cudaMemsetAsync(state_d, 0, sizeof(DecodeState), s);
 			if (dequant)
 			{
-				launch_dequant(bp, in, false, s);
-				ok = ok && last_captured_node(s, node_dequant);
+				launch_dequant(bp, in, pdl && packets, s);
+				ok = ok && last_captured_node(s, nodes.dequant);
 				timing.mark(device, s, "dequant");
 			}
 			// Programmatic launches follow a kernel only (not the clear of an inverse-only decode).
@@ -1422,7 +1437,7 @@ struct pyrowave_decoder_opaque
 				}
 				else
 					launch_idwt_level(lp[level], in, out, &band_maps[level], programmatic, s);
-				ok = ok && last_captured_node(s, dequant ? node_idwt_full[level] : node_idwt_only[level]);
+				ok = ok && last_captured_node(s, nodes.idwt[level]);
 				timing.mark(device, s, idwt_tags[level]);
 			}
 			ok = graph.end(s, key) && ok;
@@ -1438,15 +1453,23 @@ struct pyrowave_decoder_opaque
 			DecodeInput din = in;
 			PlaneOutput pout = out;
 			bool ok = true;
+			if (packets)
+			{
+				PacketParams pp = *packets;
+				// One CTA per packet, so the grids follow the call.
+				nodes.packet_tables.params.gridDim.x = nodes.packet_blocks.params.gridDim.x = unsigned(pp.count);
+				ok = set_kernel_args(graph.exec, nodes.packet_tables, pp) &&
+				     set_kernel_args(graph.exec, nodes.packet_blocks, pp);
+			}
 			if (dequant)
 			{
-				ok = set_kernel_args(graph.exec, node_dequant, bp, din);
+				ok = ok && set_kernel_args(graph.exec, nodes.dequant, bp, din);
 			}
 			for (int level = kLevels - 1; level >= 0 && ok; level--)
 			{
 				const bool pair = pairs(level);
 				level -= pair ? 1 : 0;
-				const KernelNode &node = dequant ? node_idwt_full[level] : node_idwt_only[level];
+				const KernelNode &node = nodes.idwt[level];
 				ok = pair ? set_kernel_args(graph.exec, node, lp[level], lp[level + 1], din, pout)
 				          : set_kernel_args(graph.exec, node, lp[level], din, pout, band_maps[level]);
 			}
@@ -1536,7 +1559,6 @@ struct pyrowave_decoder_opaque
 		pp.first = pk_first;
 		pp.counter = pk_counter;
 		pp.status = pk_status;
-		launch_packet_assembly(pp, s);
 		DecodeInput in = {};
 		in.keys = pk_first;
 		in.payload = pp.data;
@@ -1544,7 +1566,7 @@ struct pyrowave_decoder_opaque
 		in.jobs = jobs_d;
 		in.coef32 = coef32;
 		in.coef16 = coef16;
-		if (!run(in, out, s, true))
+		if (!run(in, out, s, true, &pp))
 			return PYROWAVE_ERROR_GENERIC;
 		cudaEventRecord(pk_done, s);
 		pk_pending = true;

@@ -464,7 +464,10 @@ struct PacketParams
 };
 
 constexpr int kMaxPackets = 1 << 20;
-void launch_packet_assembly(const PacketParams &pp, cudaStream_t stream);
+// The two passes of the assembly, one CTA per packet. The second starts early
+// after the first, and lets the dequantiser start early.
+void launch_packet_tables(const PacketParams &pp, cudaStream_t stream);
+void launch_packet_blocks(const PacketParams &pp, cudaStream_t stream);
 
 // Batched launchers: `cta_map` holds one batch_cta() word per CTA.
 // large_ctas selects the 1024-thread variant of a level; `maps` (may be null)

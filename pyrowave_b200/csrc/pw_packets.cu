@@ -550,6 +550,7 @@ __global__ void __launch_bounds__(256) packet_blocks_kernel(const PacketParams p
 	uint32_t first = 0, size = 0;
 	const bool ok = packet_span(pp, p, first, size);
 	const uint32_t nwords = (size + 3) / 4;
+	pdl_trigger(); // the dequantiser may launch meanwhile
 	pdl_wait();
 	// One round trip: the state, the summary and the thread's first item (which
 	// need not exist, but its place does) are read before they are known to count.
@@ -599,17 +600,17 @@ __global__ void __launch_bounds__(256) packet_blocks_kernel(const PacketParams p
 
 } // namespace
 
-void launch_packet_assembly(const PacketParams &pp, cudaStream_t stream)
+void launch_packet_tables(const PacketParams &pp, cudaStream_t stream)
 {
 	cudaFuncSetAttribute(packet_tables_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPacketSmemBytes));
-	{
-		LaunchConfig lc(dim3(pp.count), dim3(kPacketThreads), stream, false);
-		lc.cfg.dynamicSmemBytes = kPacketSmemBytes;
-		cudaLaunchKernelEx(&lc.cfg, packet_tables_kernel, pp);
-	}
-	{
-		LaunchConfig lc(dim3(pp.count), dim3(256), stream, true);
-		cudaLaunchKernelEx(&lc.cfg, packet_blocks_kernel, pp);
-	}
+	LaunchConfig lc(dim3(pp.count), dim3(kPacketThreads), stream, false);
+	lc.cfg.dynamicSmemBytes = kPacketSmemBytes;
+	cudaLaunchKernelEx(&lc.cfg, packet_tables_kernel, pp);
+}
+
+void launch_packet_blocks(const PacketParams &pp, cudaStream_t stream)
+{
+	LaunchConfig lc(dim3(pp.count), dim3(256), stream, true);
+	cudaLaunchKernelEx(&lc.cfg, packet_blocks_kernel, pp);
 }
 } // namespace pw
