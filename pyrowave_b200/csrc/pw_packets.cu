@@ -403,43 +403,52 @@ __device__ void scan_packets(const PacketParams &pp)
 		s_last_total = 0;
 		s_invalid = 0;
 	}
-	// This thread's packets composed, then a scan over threads: within each
-	// warp by shuffles, then over the warp totals. Warps past the last packet
-	// hold the identity.
+	// This thread's packets composed.
 	const bool active = warp * 32 * per < n; // uniform over the warp
 	const int warps = (n + 32 * per - 1) / (32 * per);
 	unsigned long long incl = kIdentityMap;
 	for (int p = p0; p < p1; p++)
 		incl = compose(incl, packet_map(pp, p));
-	if (active)
+	// The packets of one frame have one map, which changes nothing the second
+	// time: no scan (1080p in 51 packets: 40.3 -> 39.7 us with the decode).
+	const unsigned long long one = packet_map(pp, 0);
+	const bool alike = __syncthreads_and(per == 1 && (t >= n || incl == one) && compose(one, one) == one);
+	unsigned long long before = t == 0 ? kIdentityMap : one, all = one;
+	if (!alike)
 	{
+		// A scan over threads: within each warp by shuffles, then over the warp
+		// totals. Warps past the last packet hold the identity.
+		if (active)
+		{
 #pragma unroll
-		for (int off = 1; off < 32; off *= 2)
-		{
-			const unsigned long long other = __shfl_up_sync(0xffffffffu, incl, off);
-			if (lane >= off)
-				incl = compose(other, incl);
+			for (int off = 1; off < 32; off *= 2)
+			{
+				const unsigned long long other = __shfl_up_sync(0xffffffffu, incl, off);
+				if (lane >= off)
+					incl = compose(other, incl);
+			}
 		}
-	}
-	if (lane == 31)
-		s_warp[warp] = incl;
-	__syncthreads();
-	if (warp == 0)
-	{
-		unsigned long long w = s_warp[lane];
-		for (int off = 1; off < warps; off *= 2)
+		if (lane == 31)
+			s_warp[warp] = incl;
+		__syncthreads();
+		if (warp == 0)
 		{
-			const unsigned long long other = __shfl_up_sync(0xffffffffu, w, off);
-			if (lane >= off)
-				w = compose(other, w);
+			unsigned long long w = s_warp[lane];
+			for (int off = 1; off < warps; off *= 2)
+			{
+				const unsigned long long other = __shfl_up_sync(0xffffffffu, w, off);
+				if (lane >= off)
+					w = compose(other, w);
+			}
+			s_warp[lane] = w; // inclusive over the active warps
 		}
-		s_warp[lane] = w; // inclusive over the active warps
+		__syncthreads();
+		unsigned long long excl = active ? __shfl_up_sync(0xffffffffu, incl, 1) : kIdentityMap;
+		if (lane == 0)
+			excl = kIdentityMap;
+		before = compose(warp == 0 ? kIdentityMap : s_warp[warp - 1], excl);
+		all = s_warp[warps - 1];
 	}
-	__syncthreads();
-	unsigned long long excl = active ? __shfl_up_sync(0xffffffffu, incl, 1) : kIdentityMap;
-	if (lane == 0)
-		excl = kIdentityMap;
-	const unsigned long long before = compose(warp == 0 ? kIdentityMap : s_warp[warp - 1], excl);
 	// State before each of this thread's packets (the maps applied to "no
 	// sequence"); the last restart and the last accepted header (ordered by
 	// packet, then item: 1 + packet << 16 | item).
@@ -469,7 +478,7 @@ __device__ void scan_packets(const PacketParams &pp)
 	if (t == 0)
 	{
 		PacketStatus st = {};
-		const uint32_t final_state = n > 0 ? map_at(s_warp[warps - 1], kNoneState) : kNoneState;
+		const uint32_t final_state = map_at(all, kNoneState);
 		st.sequence = final_state == kNoneState ? 0xffffffffu : final_state - 1;
 		st.invalid_packets = s_invalid;
 		const unsigned long long lr = s_last_restart;
