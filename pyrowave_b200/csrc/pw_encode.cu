@@ -1,5 +1,5 @@
 // Encoder kernels for sm_100a: fused forward CDF 9/7 level + quantiser + RD
-// analysis, the single-CTA rate-control resolve, and block packing.
+// analysis, the rate-control resolve (one cluster of CTAs), and block packing.
 //
 // Reference behaviour followed (file:line in the reference tree):
 //   forward level      shaders/dwt.comp:38-234 (tile + apron, H then V lifting)
@@ -423,7 +423,7 @@ template <int kRowsIn> struct DwtSharedT
 
 // Work split of the forward level for a CTA of kThreads threads. Whole tiles
 // of large levels favour few instructions (long lifting segments: 24 samples
-// lifted for 16 kept), stripes and 1024-thread CTAs a short chain.
+// lifted for 16 kept), stripes and the batch's 1024-thread CTAs a short chain.
 template <int kThreads, int kStripes> struct DwtSplit
 {
 	static constexpr bool kShort = kThreads >= 1024 || kStripes > 1;

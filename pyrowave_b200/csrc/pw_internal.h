@@ -401,10 +401,10 @@ void launch_batch_persistent(const BatchRunParams &rp, int ctas, cudaStream_t st
 // the first of a sequence may start early (programmatic dependent launch):
 // kernels wait for their predecessor with griddepcontrol before touching
 // global memory.
-// Levels with fewer tiles than this (all components) are "small": their
-// transforms run 1024-thread CTAs, and the encoder quantises their bands in one
-// launch across the whole GPU after the last level instead of inside the
-// transform of each level.
+// Levels with fewer tiles than this (all components) are "small": four CTAs
+// transform a tile (one stripe of rows each), and the encoder quantises their
+// bands in one launch across the whole GPU after the last level instead of
+// inside the transform of each level.
 constexpr int kSmallLevelTiles = 256;
 // CTAs per tile of a small transform-only level (row stripes of the tile).
 constexpr int kDwtStripeCtas = 4;
