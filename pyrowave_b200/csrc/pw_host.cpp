@@ -19,6 +19,7 @@
 
 #include <algorithm>
 #include <array>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -453,7 +454,9 @@ struct pyrowave_device_opaque
 {
 	int cuda_device = 0;
 	cudaStream_t stream = nullptr;
-	bool stage_timing = false;
+	// Any thread may switch it; a call reads it once, since the launches it captures,
+	// their arguments and the events between them all follow from it.
+	std::atomic<bool> stage_timing{false};
 	std::mutex lock;
 	std::vector<StageTimer> timers;
 
@@ -490,9 +493,9 @@ struct StageEvents
 	bool created = false;
 
 	// Outside stream capture: create the events once timing is on.
-	void prepare(pyrowave_device_opaque *dev)
+	void prepare(bool timed)
 	{
-		if (!dev->stage_timing || created)
+		if (!timed || created)
 			return;
 		for (auto &e : ev)
 			cuda_ok(cudaEventCreate(&e), "cudaEventCreate");
@@ -509,25 +512,25 @@ struct StageEvents
 		else
 			cuda_ok(cudaEventRecord(e, s), "cudaEventRecord");
 	}
-	void begin(pyrowave_device_opaque *dev, cudaStream_t s, bool in_capture = true)
+	void begin(bool timed, cudaStream_t s, bool in_capture = true)
 	{
-		if (!dev->stage_timing || !created)
+		if (!timed || !created)
 			return;
 		count = 0;
 		captured = in_capture;
 		record(s, ev[0]);
 	}
-	void mark(pyrowave_device_opaque *dev, cudaStream_t s, const char *tag)
+	void mark(bool timed, cudaStream_t s, const char *tag)
 	{
-		if (!dev->stage_timing || !created || count >= kMax)
+		if (!timed || !created || count >= kMax)
 			return;
 		tags[count++] = tag;
 		record(s, ev[count]);
 	}
 	// The events of the captured sequence were launched (they are graph nodes).
-	void launched(pyrowave_device_opaque *dev)
+	void launched(bool timed)
 	{
-		if (dev->stage_timing && created && count > 0)
+		if (timed && created && count > 0)
 			pending = true;
 	}
 	void collect(pyrowave_device_opaque *dev)
@@ -936,9 +939,10 @@ struct pyrowave_encoder_opaque
 		sequence_count = (sequence_count + 1) & 7u;
 		EncodeBuffers b = buffers();
 		b.tile_done = tile_done();
+		const bool timed = device->stage_timing;
 		timing.collect(device);
-		timing.prepare(device);
-		const uint64_t key = uint64_t(stream_capacity) | (device->stage_timing ? (1ull << 40) : 0ull);
+		timing.prepare(timed);
+		const uint64_t key = uint64_t(stream_capacity) | (timed ? (1ull << 40) : 0ull);
 		if (!graph.valid() || graph.key != key)
 		{
 			// Capture the frame's kernel sequence once (pyrowave_encoder.cpp:1153-1183:
@@ -946,10 +950,10 @@ struct pyrowave_encoder_opaque
 			if (!graph.begin(s))
 				return PYROWAVE_ERROR_GENERIC;
 			bool ok = true;
-			timing.begin(device, s);
+			timing.begin(timed, s);
 			cudaMemsetAsync(rc, 0, rc_bytes(), s);
 			static const char *const dwt_tags[kLevels] = {"dwt0", "dwt1", "dwt2", "dwt3", "dwt4"};
-			const bool pdl = !device->stage_timing; // event nodes between kernels break programmatic edges
+			const bool pdl = !timed; // event nodes between kernels break programmatic edges
 			// The small levels (few tiles each) transform only, each level one launch;
 			// one launch then quantises all their blocks, so no level's quantiser
 			// waits on the critical path of the transforms.
@@ -957,18 +961,18 @@ struct pyrowave_encoder_opaque
 			{
 				launch_dwt_forward_level(lp[level], in, b, level < small_level, pdl && level > 0, s);
 				ok = ok && last_captured_node(s, node_dwt[level]);
-				timing.mark(device, s, dwt_tags[level]);
+				timing.mark(timed, s, dwt_tags[level]);
 			}
 			if (small_blocks > 0)
 			{
 				launch_quant_pretransformed(bp, b, small_blocks, pdl, s);
-				timing.mark(device, s, "quant");
+				timing.mark(timed, s, "quant");
 			}
 			launch_resolve(dataflow_resolve_params(target_words), b, s);
 			ok = ok && last_captured_node(s, node_resolve);
-			timing.mark(device, s, "resolve");
+			timing.mark(timed, s, "resolve");
 			launch_pack(bp, b, s);
-			timing.mark(device, s, "pack");
+			timing.mark(timed, s, "pack");
 			ok = graph.end(s, key) && ok;
 			if (!ok)
 			{
@@ -997,7 +1001,7 @@ struct pyrowave_encoder_opaque
 		}
 		if (!cuda_ok(cudaGraphLaunch(graph.exec, s), "cudaGraphLaunch"))
 			return PYROWAVE_ERROR_GENERIC;
-		timing.launched(device);
+		timing.launched(timed);
 		cudaEventRecord(encoded, s);
 		has_device_frame = true;
 		return PYROWAVE_SUCCESS;
@@ -1382,9 +1386,9 @@ struct pyrowave_decoder_opaque
 	// Whether inverse level `level` shares a launch with the next finer one: both
 	// small (stripes), and the finer one has every component. With stage timing
 	// every level is a launch of its own.
-	bool pairs(int level) const
+	bool pairs(int level, bool timed) const
 	{
-		return !device->stage_timing && level % 2 == 0 && level >= 2 && level_tiles(g, level) < kSmallLevelTiles &&
+		return !timed && level % 2 == 0 && level >= 2 && level_tiles(g, level) < kSmallLevelTiles &&
 		       level_tiles(g, level - 1) < kSmallLevelTiles;
 	}
 
@@ -1396,11 +1400,12 @@ struct pyrowave_decoder_opaque
 		DecodeInput in = in_args;
 		in.error = error_d;
 		in.state = state_d;
+		const bool timed = device->stage_timing;
 		timing.collect(device);
-		timing.prepare(device);
+		timing.prepare(timed);
 		DecodeGraph &nodes = packets ? graph_packets : dequant ? graph_full : graph_idwt;
 		CapturedGraph &graph = nodes.graph;
-		const uint64_t key = device->stage_timing ? 1ull : 0ull;
+		const uint64_t key = timed ? 1ull : 0ull;
 		if (!graph.valid() || graph.key != key)
 		{
 			if (!graph.begin(s))
@@ -1413,8 +1418,8 @@ struct pyrowave_decoder_opaque
 				launch_packet_blocks(*packets, s);
 				ok = ok && last_captured_node(s, nodes.packet_blocks);
 			}
-			timing.begin(device, s);
-			const bool pdl = !device->stage_timing; // event nodes between kernels break programmatic edges
+			timing.begin(timed, s);
+			const bool pdl = !timed; // event nodes between kernels break programmatic edges
 			// The dequantiser clears the decode state before any inverse level runs;
 			// without it the graph starts with a clear of its own.
 			if (!dequant)
@@ -1423,14 +1428,14 @@ struct pyrowave_decoder_opaque
 			{
 				launch_dequant(bp, in, pdl && packets, s);
 				ok = ok && last_captured_node(s, nodes.dequant);
-				timing.mark(device, s, "dequant");
+				timing.mark(timed, s, "dequant");
 			}
 			// Programmatic launches follow a kernel only (not the clear of an inverse-only decode).
 			static const char *const idwt_tags[kLevels] = {"idwt0", "idwt1", "idwt2", "idwt3", "idwt4"};
 			for (int level = kLevels - 1; level >= 0; level--)
 			{
 				const bool programmatic = pdl && (dequant || level < kLevels - 1);
-				if (pairs(level))
+				if (pairs(level, timed))
 				{
 					level--;
 					launch_idwt_pair(lp[level], lp[level + 1], in, out, programmatic, s);
@@ -1438,7 +1443,7 @@ struct pyrowave_decoder_opaque
 				else
 					launch_idwt_level(lp[level], in, out, &band_maps[level], programmatic, s);
 				ok = ok && last_captured_node(s, nodes.idwt[level]);
-				timing.mark(device, s, idwt_tags[level]);
+				timing.mark(timed, s, idwt_tags[level]);
 			}
 			ok = graph.end(s, key) && ok;
 			if (!ok)
@@ -1467,7 +1472,7 @@ struct pyrowave_decoder_opaque
 			}
 			for (int level = kLevels - 1; level >= 0 && ok; level--)
 			{
-				const bool pair = pairs(level);
+				const bool pair = pairs(level, timed);
 				level -= pair ? 1 : 0;
 				const KernelNode &node = nodes.idwt[level];
 				ok = pair ? set_kernel_args(graph.exec, node, lp[level], lp[level + 1], din, pout)
@@ -1482,7 +1487,7 @@ struct pyrowave_decoder_opaque
 		}
 		if (!cuda_ok(cudaGraphLaunch(graph.exec, s), "cudaGraphLaunch"))
 			return false;
-		timing.launched(device);
+		timing.launched(timed);
 		cudaEventRecord(decode_done, s);
 		decode_pending = true;
 		decoded_frame_for_current_sequence = true;
@@ -2343,17 +2348,18 @@ pyrowave_result pyrowave_cuda_encoder_transform(pyrowave_encoder encoder, const 
 	cudaStream_t s = pick_stream(encoder->device, stream);
 	pyrowave_device_opaque *dev = encoder->device;
 	StageEvents &timing = encoder->timing;
+	const bool timed = dev->stage_timing;
 	timing.collect(dev);
-	timing.prepare(dev);
-	timing.begin(dev, s, false);
+	timing.prepare(timed);
+	timing.begin(timed, s, false);
 	static const char *const tags[kLevels] = {"xdwt0", "xdwt1", "xdwt2", "xdwt3", "xdwt4"};
 	const EncodeBuffers b = encoder->buffers();
 	for (int level = 0; level < kLevels; level++)
 	{
-		launch_dwt_forward_level(encoder->lp[level], in, b, false, level > 0 && !dev->stage_timing, s);
-		timing.mark(dev, s, tags[level]);
+		launch_dwt_forward_level(encoder->lp[level], in, b, false, level > 0 && !timed, s);
+		timing.mark(timed, s, tags[level]);
 	}
-	timing.launched(dev);
+	timing.launched(timed);
 	return launches_ok("kernel launch") ? PYROWAVE_SUCCESS : PYROWAVE_ERROR_GENERIC;
 }
 
