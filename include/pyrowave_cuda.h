@@ -197,7 +197,7 @@ PYROWAVE_PUBLIC_API pyrowave_result pyrowave_cuda_decoder_decode_blocks16(pyrowa
  * (pyrowave_decoder.cpp:126-262), then pyrowave_decoder_decode_gpu_buffer.
  * `data` holds the packets in device memory (4-byte aligned, at most 4 GiB);
  * `packets` is a device array of `count` {offset, size} byte ranges of `data`,
- * in push order, each offset a multiple of 4. The sequence rules of the
+ * in push order, each offset a multiple of 4; ranges may overlap. The sequence rules of the
  * reference parser apply (a newer sequence restarts the frame, packets of an
  * older one are ignored from that point of the packet on, the first copy of a
  * block wins); blocks not received decode as zero. A packet the host parser

@@ -1123,8 +1123,8 @@ struct pyrowave_decoder_opaque
 	uint8_t *pk_state = nullptr;
 	uint32_t *pk_summaries = nullptr;
 	size_t pk_capacity = 0; // packets
-	uint32_t *pk_items = nullptr;
-	size_t pk_items_capacity = 0; // words of each half (positions, blocks)
+	unsigned long long *pk_items = nullptr;
+	size_t pk_items_capacity = 0; // items
 	unsigned long long *pk_first = nullptr;
 	PacketStatus *pk_status = nullptr;
 	PacketStatus *pk_status_h = nullptr;
@@ -1542,7 +1542,7 @@ struct pyrowave_decoder_opaque
 			cudaStreamSynchronize(s);
 			dev_free(pk_items);
 			const size_t cap = std::max<size_t>(data_words, 1 << 16);
-			pk_items = dev_alloc<uint32_t>(2 * cap, ok);
+			pk_items = dev_alloc<unsigned long long>(cap, ok);
 			pk_items_capacity = ok ? cap : 0;
 		}
 		if (!ok)
@@ -1560,7 +1560,6 @@ struct pyrowave_decoder_opaque
 		pp.state_before = pk_state;
 		pp.summaries = pk_summaries;
 		pp.items = pk_items;
-		pp.item_blocks = pk_items + pk_items_capacity;
 		pp.first = pk_first;
 		pp.counter = pk_counter;
 		pp.status = pk_status;

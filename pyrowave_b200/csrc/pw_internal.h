@@ -456,8 +456,7 @@ struct PacketParams
 	uint32_t *tables;                 // count x 9 x {state | error << 4 | restart << 8, total}
 	uint8_t *state_before;            // count
 	uint32_t *summaries;              // count x 8 words: each packet's item summary
-	uint32_t *items;                  // data_bytes / 4: packet p's item positions at its own first word on
-	uint32_t *item_blocks;            // likewise the items' block indices, ~0 for a sequence header
+	unsigned long long *items;        // data_bytes / 4: packet p's items (item_record) at its own first word on
 	unsigned long long *first;        // block_count: smallest (packet, item, word offset) key, ~0 = missing
 	uint32_t *counter;                // CTAs of the table pass done (zero between calls)
 	PacketStatus *status;

@@ -208,8 +208,19 @@ __device__ __forceinline__ ItemInfo classify(uint32_t w0, uint32_t w1, uint32_t 
 	return it;
 }
 
+// A listed item in one word, so that its parts stay together: its position, its
+// number in the packet and its block. Packets whose byte ranges overlap share
+// slots of the list; a slot that holds another number than its reader's was
+// stored for a packet that starts elsewhere (with the same number, for one that
+// starts at the same word, where the items are the same).
+__device__ __forceinline__ unsigned long long item_record(uint32_t pos, uint32_t k, uint32_t block)
+{
+	return (unsigned long long)block << 32 | (k << 16 | pos);
+}
+static_assert(kFastWords <= 0x10000, "positions and item numbers in 16 bits");
+
 // Stages the packet (nwords <= kFastWords), lists its items in pp.items and
-// pp.item_blocks and fills the item summary. Every thread of the CTA calls it.
+// fills the item summary. Every thread of the CTA calls it.
 __device__ void discover_items(PacketSmem &sm, ItemSummary &sum, const PacketParams &pp, uint32_t first,
                                uint32_t size, uint32_t nwords)
 {
@@ -298,8 +309,7 @@ __device__ void discover_items(PacketSmem &sm, ItemSummary &sum, const PacketPar
 			continue;
 		}
 		const ItemInfo it = classify(sm.words[q], sm.words[q + 1], size - 4 * q, pp);
-		pp.items[first + k] = q;
-		pp.item_blocks[first + k] = it.header ? kNoBlock : it.block;
+		pp.items[first + k] = item_record(q, k, it.header ? kNoBlock : it.block);
 		if (it.error)
 			sum.error = k << 2 | it.error;
 		else if (it.header)
@@ -566,12 +576,9 @@ __global__ void __launch_bounds__(256) packet_blocks_kernel(const PacketParams p
 	const uint32_t seq = __ldcg(&pp.status->sequence);
 	const uint32_t state = pp.state_before[p];
 	const ItemSummary sum = reinterpret_cast<const ItemSummary *>(pp.summaries)[p];
-	uint32_t pos = 0, block = kNoBlock;
+	unsigned long long rec = 0;
 	if (ok && threadIdx.x < nwords)
-	{
-		pos = __ldcg(pp.items + first + threadIdx.x);
-		block = __ldcg(pp.item_blocks + first + threadIdx.x);
-	}
+		rec = __ldcg(pp.items + first + threadIdx.x);
 	if (!ok || seq == 0xffffffffu || uint32_t(p) < rp)
 		return; // uniform over the CTA
 	uint32_t fresh = 0; // blocks this thread saw first
@@ -582,24 +589,28 @@ __global__ void __launch_bounds__(256) packet_blocks_kernel(const PacketParams p
 		if (atomicMin(pp.first + b, key) == kNoKey)
 			fresh++;
 	};
+	bool walk = true;
 	if (sum.fast && sum.seq_min == sum.seq_max)
 	{
 		bool accepts;
 		(void)uniform_walk(sum, state, accepts);
 		const uint32_t err_item = sum.error == ~0u ? ~0u : sum.error >> 2;
 		const uint32_t n = accepts ? min(sum.nitems, err_item) : 0u;
+		bool lost = false;
 		for (uint32_t k = threadIdx.x; k < n; k += blockDim.x)
 		{
 			if (k >= blockDim.x)
-			{
-				pos = __ldcg(pp.items + first + k);
-				block = __ldcg(pp.item_blocks + first + k);
-			}
-			if (pos + 1 < nwords && block < uint32_t(pp.block_count)) // not a sequence header
+				rec = __ldcg(pp.items + first + k);
+			const uint32_t pos = uint32_t(rec) & 0xffffu, block = uint32_t(rec >> 32);
+			if (((uint32_t(rec) >> 16) & 0xffffu) != k)
+				lost = true;
+			else if (pos + 1 < nwords && block < uint32_t(pp.block_count)) // not a sequence header
 				keep(block, pos, k);
 		}
+		walk = __syncthreads_or(lost);
 	}
-	else if (threadIdx.x == 0)
+	// Item by item (proposing a block a second time changes nothing).
+	if (walk && threadIdx.x == 0)
 		walk_packet([&](uint32_t i) { return i < nwords ? __ldg(pp.data + first + i) : 0u; }, size, state, pp, keep);
 	fresh = __reduce_add_sync(0xffffffffu, fresh);
 	if ((threadIdx.x & 31) == 0 && fresh)
