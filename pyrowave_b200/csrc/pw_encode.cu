@@ -890,22 +890,30 @@ __device__ __forceinline__ void dwt_forward_body(DwtSharedT<DwtSplit<kThreads, k
 				e[4 + 2 * k] = f2_mul_rn(e[4 + 2 * k], f2_pack(kInvK, kInvK));
 				e[5 + 2 * k] = f2_mul_rn(e[5 + 2 * k], f2_pack(kK, kK));
 			}
-			if (!whole || (kHalf && (L.fp16 || L.stage16)))
+			if (kHalf && (L.fp16 || L.stage16))
 			{
 #pragma unroll
 				for (int k = 0; k < 2 * kPairs; k++)
 				{
-					float a[2];
-					f2_unpack(e[4 + k], a[0], a[1]);
+					float lo, hi;
+					f2_unpack(e[4 + k], lo, hi);
+					e[4 + k] = f2_pack(round_to_half(lo), round_to_half(hi));
+				}
+			}
+			if (!whole)
+			{
+				// By masks made once: compared sample by sample, these spilled in the batch's
+				// persistent kernel, and a partial tile's pass took 5.1 K cycles instead of 2.1 K.
+				const uint32_t m0 = gx < L.width ? ~0u : 0u, m1 = gx + 1 < L.width ? ~0u : 0u;
+				const int rows = L.height - gy;
 #pragma unroll
-					for (int i = 0; i < 2; i++)
-					{
-						if (kHalf && (L.fp16 || L.stage16))
-							a[i] = round_to_half(a[i]);
-						if (gx + i >= L.width || gy + (k >> 1) >= L.height)
-							a[i] = 0.0f;
-					}
-					e[4 + k] = f2_pack(a[0], a[1]);
+				for (int k = 0; k < 2 * kPairs; k++)
+				{
+					const bool inside = (k >> 1) < rows;
+					float lo, hi;
+					f2_unpack(e[4 + k], lo, hi);
+					e[4 + k] = f2_pack(__uint_as_float(inside ? __float_as_uint(lo) & m0 : 0u),
+					                   __uint_as_float(inside ? __float_as_uint(hi) & m1 : 0u));
 				}
 			}
 			if (kHalf && L.fp16)
