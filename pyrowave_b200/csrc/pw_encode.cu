@@ -11,6 +11,8 @@
 //   packetize layout   pyrowave_encoder.cpp:1048-1115
 #include "pw_decode_body.cuh"
 
+#include <algorithm>
+
 namespace pw
 {
 namespace
@@ -1959,8 +1961,10 @@ __device__ __forceinline__ BatchShared &batch_shared() { return *reinterpret_cas
 
 // Each stage body is its own function (not inlined into the loop), so that
 // register allocation happens per stage, as in the single-frame kernels; each
-// reaches the shared storage through the kernel's own symbol.
-__device__ __noinline__ void batch_forward_item(int level, int small_level, int local)
+// reaches the shared storage through the kernel's own symbol. The two kernels
+// have functions of their own: with functions that both called, one kernel's
+// decoded samples were off by one in places (nvcc 12.9).
+template <bool kManyItems> __device__ __noinline__ void batch_forward_item(int level, int small_level, int local)
 {
 	BatchShared &sh = batch_shared();
 	const int per_comp = sh.prm.lp.L.tiles_x * sh.prm.lp.L.tiles_y;
@@ -1968,31 +1972,31 @@ __device__ __noinline__ void batch_forward_item(int level, int small_level, int 
 	                                                    local % per_comp, local / per_comp);
 }
 
-__device__ __noinline__ void batch_quant_item(int small_blocks, int local)
+template <bool kManyItems> __device__ __noinline__ void batch_quant_item(int small_blocks, int local)
 {
 	BatchShared &sh = batch_shared();
 	quant_blocks_body<1, 2>(sh.prm.bp, sh.eb, 0, small_blocks, local, sh.u.quant.tile, sh.u.quant.q, sh.u.quant.scales);
 }
 
-__device__ __noinline__ void batch_resolve_item(int slice, int slices)
+template <bool kManyItems> __device__ __noinline__ void batch_resolve_item(int slice, int slices)
 {
 	BatchShared &sh = batch_shared();
 	resolve_body(sh.prm.rp, sh.eb, slice, slices);
 }
 
-__device__ __noinline__ void batch_pack_item(int blk, int warp)
+template <bool kManyItems> __device__ __noinline__ void batch_pack_item(int blk, int warp)
 {
 	BatchShared &sh = batch_shared();
 	pack_body(sh.u.pack[warp], sh.prm.bp, sh.eb, blk);
 }
 
-__device__ __noinline__ void batch_dequant_item(int blk, int warp)
+template <bool kManyItems> __device__ __noinline__ void batch_dequant_item(int blk, int warp)
 {
 	BatchShared &sh = batch_shared();
 	dequant_body(sh.u.deq[warp], sh.prm.bp, sh.di, blk, blk == 0);
 }
 
-__device__ __noinline__ void batch_inverse_item(int local)
+template <bool kManyItems> __device__ __noinline__ void batch_inverse_item(int local)
 {
 	BatchShared &sh = batch_shared();
 	const int per_comp = sh.prm.lp.L.tiles_x * sh.prm.lp.L.tiles_y;
@@ -2000,13 +2004,19 @@ __device__ __noinline__ void batch_inverse_item(int local)
 	                                   local / per_comp);
 }
 
+template <bool kManyItems>
 __global__ void __launch_bounds__(kBatchPersistentThreads, 4) batch_persistent_kernel(const BatchRunParams rp)
 {
 	BatchShared &sh = batch_shared();
 	// Thread 0 holds the CTA's next ticket, taken while the current item runs,
-	// so the ticket's round trip overlaps the work. Tickets are still processed
-	// in increasing order by every CTA, and an item only waits for items with
-	// smaller tickets, so every wait still ends.
+	// so the ticket's round trip overlaps the work. Without kManyItems a CTA that
+	// waits at a gate takes it only once items of the gating stage have finished:
+	// taken while idle, it would put two items of one stage on this CTA and none on
+	// another (one 1080p frame, encode + decode: 247 us, now 202). With kManyItems,
+	// two items per CTA and more in some stage, it is taken at once (twelve mixed
+	// frames: 1702 us, 1733 waiting for the gate first). Tickets are still
+	// processed in increasing order by every CTA, and an item only waits for items
+	// with smaller tickets, so every wait still ends.
 	int next = 0;
 	if (threadIdx.x == 0)
 		next = int(atomicAdd(rp.ticket, 1u));
@@ -2018,7 +2028,7 @@ __global__ void __launch_bounds__(kBatchPersistentThreads, 4) batch_persistent_k
 		const int item = sh.item;
 		if (item >= rp.nwork)
 			return;
-		if (threadIdx.x == 0)
+		if (kManyItems && threadIdx.x == 0)
 			next = int(atomicAdd(rp.ticket, 1u));
 		const uint32_t w = __ldg(rp.work + item);
 		const int f = int(w >> 24), stage = int((w >> kBatchLocalBits) & 31u);
@@ -2026,14 +2036,20 @@ __global__ void __launch_bounds__(kBatchPersistentThreads, 4) batch_persistent_k
 		const BatchFrame &fr = rp.frames[f];
 		if (threadIdx.x == 0)
 		{
+			bool taken = kManyItems;
 			const uint32_t gate = __ldg(rp.gates + f * kBatchStages + stage);
 			if (gate != kNoGate)
 			{
 				const uint32_t *count = rp.done + f * kBatchStages + (gate >> 24);
 				const uint32_t target = gate & 0xffffffu;
-				uint32_t spins = 0;
-				while (ld_acquire_u32(count) < target)
+				uint32_t spins = 0, finished;
+				while ((finished = ld_acquire_u32(count)) < target)
 				{
+					if (finished != 0 && !taken)
+					{
+						next = int(atomicAdd(rp.ticket, 1u));
+						taken = true;
+					}
 					if (++spins > kBatchWaitSpins)
 					{
 						atomicOr(&fr.eb.rc->error, kErrorLevelWait);
@@ -2042,6 +2058,8 @@ __global__ void __launch_bounds__(kBatchPersistentThreads, 4) batch_persistent_k
 					__nanosleep(64);
 				}
 			}
+			if (!taken)
+				next = int(atomicAdd(rp.ticket, 1u));
 		}
 		if (stage < kStageQuant)
 		{
@@ -2073,25 +2091,25 @@ __global__ void __launch_bounds__(kBatchPersistentThreads, 4) batch_persistent_k
 		__syncthreads();
 		const int warp = int(threadIdx.x) >> 5;
 		if (stage < kStageQuant)
-			batch_forward_item(stage - kStageDwt0, rp.small_level, local);
+			batch_forward_item<kManyItems>(stage - kStageDwt0, rp.small_level, local);
 		else if (stage == kStageQuant)
-			batch_quant_item(fr.small_blocks, local);
+			batch_quant_item<kManyItems>(fr.small_blocks, local);
 		else if (stage == kStageResolve)
-			batch_resolve_item(local, fr.slices);
+			batch_resolve_item<kManyItems>(local, fr.slices);
 		else if (stage == kStagePack)
 		{
 			const int blk = local * kBatchBlockItem + warp;
 			if (blk < fr.block_count)
-				batch_pack_item(blk, warp);
+				batch_pack_item<kManyItems>(blk, warp);
 		}
 		else if (stage == kStageDequant)
 		{
 			const int blk = local * kBatchBlockItem + warp;
 			if (blk < fr.block_count)
-				batch_dequant_item(blk, warp);
+				batch_dequant_item<kManyItems>(blk, warp);
 		}
 		else
-			batch_inverse_item(local);
+			batch_inverse_item<kManyItems>(local);
 		__syncthreads();
 		if (threadIdx.x == 0)
 		{
@@ -2103,31 +2121,40 @@ __global__ void __launch_bounds__(kBatchPersistentThreads, 4) batch_persistent_k
 
 } // namespace
 
+namespace
+{
+template <bool kManyItems> int persistent_ctas_per_sm()
+{
+	cudaFuncSetAttribute(batch_persistent_kernel<kManyItems>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+	                     int(sizeof(BatchShared)));
+	int n = 0;
+	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_persistent_kernel<kManyItems>, kBatchPersistentThreads,
+	                                                  sizeof(BatchShared)) != cudaSuccess ||
+	    n < 1)
+	{
+		(void)cudaGetLastError();
+		n = 1;
+	}
+	return n;
+}
+} // namespace
+
 int batch_persistent_max_ctas_per_sm()
 {
 	static int cached = 0;
 	if (!cached)
-	{
-		cudaFuncSetAttribute(batch_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-		                     int(sizeof(BatchShared)));
-		int n = 0;
-		if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_persistent_kernel, kBatchPersistentThreads,
-		                                                  sizeof(BatchShared)) != cudaSuccess ||
-		    n < 1)
-		{
-			(void)cudaGetLastError();
-			n = 1;
-		}
-		cached = n;
-	}
+		cached = std::min(persistent_ctas_per_sm<false>(), persistent_ctas_per_sm<true>());
 	return cached;
 }
 
-// The kernel's shared-memory attribute is set by batch_persistent_max_ctas_per_sm,
+// The kernels' shared-memory attribute is set by batch_persistent_max_ctas_per_sm,
 // which the batch calls before any launch (outside stream capture).
-void launch_batch_persistent(const BatchRunParams &rp, int ctas, cudaStream_t stream)
+void launch_batch_persistent(const BatchRunParams &rp, bool many_items, int ctas, cudaStream_t stream)
 {
-	batch_persistent_kernel<<<ctas, kBatchPersistentThreads, sizeof(BatchShared), stream>>>(rp);
+	if (many_items)
+		batch_persistent_kernel<true><<<ctas, kBatchPersistentThreads, sizeof(BatchShared), stream>>>(rp);
+	else
+		batch_persistent_kernel<false><<<ctas, kBatchPersistentThreads, sizeof(BatchShared), stream>>>(rp);
 }
 
 LaunchConfig::LaunchConfig(dim3 grid, dim3 block, cudaStream_t stream, bool programmatic)

@@ -2730,6 +2730,7 @@ struct pyrowave_cuda_batch_opaque
 	// stage gates, and the ticket / finished-item counters cleared per call.
 	uint32_t *work_d[2] = {};
 	int work_n[2] = {};
+	bool many_items = false; // some stage has at least two items per CTA
 	uint32_t *gates_d = nullptr;
 	uint32_t *sync_d = nullptr; // ticket, then count x kBatchStages finished counters
 	int sm_count = 148;
@@ -2890,8 +2891,9 @@ struct pyrowave_cuda_batch_opaque
 
 	// Work lists and gates of the persistent mode: stage by stage, every frame's
 	// items (frames in index order, or largest first); an item is gated by the
-	// nearest earlier stage of its frame that has items.
-	void build_work(std::vector<uint32_t> (&work)[2], std::vector<uint32_t> &gates) const
+	// nearest earlier stage of its frame that has items. Returns the most items
+	// that a stage has over all frames.
+	size_t build_work(std::vector<uint32_t> (&work)[2], std::vector<uint32_t> &gates) const
 	{
 		std::vector<int> order(static_cast<size_t>(count));
 		for (int f = 0; f < count; f++)
@@ -2916,15 +2918,21 @@ struct pyrowave_cuda_batch_opaque
 					prev = st;
 			}
 		}
+		size_t most = 0;
 		for (int d = 0; d < 2; d++)
 		{
 			work[d].clear();
 			const int last = d ? kBatchStages : kStageDequant;
 			for (int st = 0; st < last; st++)
+			{
+				const size_t begin = work[d].size();
 				for (int f : order)
 					for (int i = 0; i < n[size_t(f)][size_t(st)]; i++)
 						work[d].push_back(batch_work(f, st, i));
+				most = std::max(most, work[d].size() - begin);
+			}
 		}
+		return most;
 	}
 
 	int persistent_ctas() const
@@ -2969,7 +2977,7 @@ struct pyrowave_cuda_batch_opaque
 		(void)batch_persistent_max_ctas_per_sm(); // kernel attributes, set outside any capture
 		bool ok = true;
 		std::vector<uint32_t> work[2], gates;
-		build_work(work, gates);
+		many_items = build_work(work, gates) >= size_t(2 * persistent_ctas());
 		for (int d = 0; d < 2; d++)
 		{
 			if (work_d[d])
@@ -3037,7 +3045,7 @@ struct pyrowave_cuda_batch_opaque
 			rp.done = sync_d + 1;
 			rp.nwork = work_n[decode ? 1 : 0];
 			rp.small_level = shape.small_level;
-			launch_batch_persistent(rp, persistent_ctas(), s);
+			launch_batch_persistent(rp, many_items, persistent_ctas(), s);
 			ok = launches_ok("kernel launch") && ok;
 			ok = graph.end(s, 0) && ok;
 			if (!ok)

@@ -395,7 +395,8 @@ struct BatchRunParams
 constexpr int kBatchPersistentThreads = 256;
 // Resident CTAs per SM of the persistent kernel (its register and shared-memory limit).
 int batch_persistent_max_ctas_per_sm();
-void launch_batch_persistent(const BatchRunParams &rp, int ctas, cudaStream_t stream);
+// many_items: some stage has at least two items, over all frames, per CTA.
+void launch_batch_persistent(const BatchRunParams &rp, bool many_items, int ctas, cudaStream_t stream);
 
 // Host-side kernel launchers (implemented in the .cu files). Every launch but
 // the first of a sequence may start early (programmatic dependent launch):
