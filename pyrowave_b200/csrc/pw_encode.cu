@@ -1952,7 +1952,11 @@ struct BatchShared
 	PlaneOutput out;
 	int item;
 };
-static_assert(sizeof(BatchShared) <= 56 * 1024, "the persistent kernel's stage storage fits four CTAs per SM");
+// Four CTAs share an SM's 228 KB; each also has the resolve's static storage
+// (8704 bytes) and 1 KB that the system reserves.
+constexpr size_t kBatchStaticShared = 8704, kSmShared = 228 * 1024;
+static_assert(4 * (sizeof(BatchShared) + kBatchStaticShared + 1024) <= kSmShared,
+              "the persistent kernel's stage storage fits four CTAs per SM");
 
 // The kernel's shared memory (dynamic: its stages' storage is a union larger
 // than a static allocation may be).
