@@ -123,10 +123,6 @@ __device__ __forceinline__ uint32_t ld_acquire_u32(const uint32_t *p)
 	return v;
 }
 
-// Orders this thread's generic-proxy view of global memory (data other CTAs
-// stored, observed through an acquire) before its later async-proxy (TMA) reads.
-__device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
-
 // Bounded wait until a counter reaches `target` (one thread). Returns false
 // when it gave up after kDataflowWaitSpins polls.
 __device__ __forceinline__ bool wait_counter(const uint32_t *c, uint32_t target)
@@ -319,34 +315,10 @@ __device__ __forceinline__ unsigned long long transpose8x8(unsigned long long x)
 	return x ^ t ^ (t << 28);
 }
 
-// The 8 coefficients of a 4x2 sub-block in the quantiser's order (i = 2 * column
-// + row) as two 4-wide row vectors: idx is the element index of (row 0, column
-// 0), a multiple of 4 (the sub-block starts on a 4-column boundary of a
+// Stores the 8 coefficients of a 4x2 sub-block in the quantiser's order (i = 2 *
+// column + row) as two 4-wide row vectors: idx is the element index of (row 0,
+// column 0), a multiple of 4 (the sub-block starts on a 4-column boundary of a
 // 32-aligned band row), pitch the row pitch in elements.
-__device__ __forceinline__ void load_subblock(const float *c32, const __half *c16, bool fp16, int64_t idx, int pitch,
-                                              float (&c)[8])
-{
-	float4 r0, r1;
-	if (fp16)
-	{
-		const uint2 a = __ldcg(reinterpret_cast<const uint2 *>(c16 + idx));
-		const uint2 b = __ldcg(reinterpret_cast<const uint2 *>(c16 + idx + pitch));
-		const float2 a0 = __half22float2(*reinterpret_cast<const __half2 *>(&a.x));
-		const float2 a1 = __half22float2(*reinterpret_cast<const __half2 *>(&a.y));
-		const float2 b0 = __half22float2(*reinterpret_cast<const __half2 *>(&b.x));
-		const float2 b1 = __half22float2(*reinterpret_cast<const __half2 *>(&b.y));
-		r0 = make_float4(a0.x, a0.y, a1.x, a1.y);
-		r1 = make_float4(b0.x, b0.y, b1.x, b1.y);
-	}
-	else
-	{
-		r0 = __ldcg(reinterpret_cast<const float4 *>(c32 + idx));
-		r1 = __ldcg(reinterpret_cast<const float4 *>(c32 + idx + pitch));
-	}
-	c[0] = r0.x, c[2] = r0.y, c[4] = r0.z, c[6] = r0.w;
-	c[1] = r1.x, c[3] = r1.y, c[5] = r1.z, c[7] = r1.w;
-}
-
 __device__ __forceinline__ void store_subblock(float *c32, __half *c16, bool fp16, int64_t idx, int pitch,
                                                const float (&c)[8])
 {
@@ -425,8 +397,6 @@ __device__ __forceinline__ float decode_quant(uint32_t code)
 	const int m = int(code & 7u);
 	return __fmul_rn(float(8 + m), __int_as_float((127 + e - 3) << 23));
 }
-
-__device__ __forceinline__ int find_msb(uint32_t v) { return v ? 31 - __clz(v) : -1; }
 
 // 8-bit quant scale per 8x8 block (wavelet_quant.comp:95-111): with target =
 // 2^e - 0.25 from the maximum's exponent, code = ceil((max / target - 0.25) * 8),

@@ -527,21 +527,21 @@ __global__ void __launch_bounds__(kPacketThreads) packet_tables_kernel(const Pac
 	}
 	if (threadIdx.x < 9)
 	{
-	const uint32_t init = threadIdx.x;
-	WalkResult r;
-	bool acc;
-	if (!ok)
-		r = WalkResult{init, kNoPos, kNoTotal, true};
-	else if (fast && sum.seq_min == sum.seq_max)
-		r = uniform_walk(sum, init, acc);
-	else if (fast)
-		r = walk_packet([&](uint32_t i) { return i < nwords ? sm.words[i] : 0u; }, size, init, pp,
-		                [](uint32_t, uint32_t, uint32_t) {});
-	else
-		r = walk_packet([&](uint32_t i) { return i < nwords ? __ldg(pp.data + first + i) : 0u; }, size, init, pp,
-		                [](uint32_t, uint32_t, uint32_t) {});
-	pp.tables[(size_t(p) * 9 + init) * 2 + 0] = r.state | (r.error ? 16u : 0u) | (r.restart << 8);
-	pp.tables[(size_t(p) * 9 + init) * 2 + 1] = r.total;
+		const uint32_t init = threadIdx.x;
+		WalkResult r;
+		bool acc;
+		if (!ok)
+			r = WalkResult{init, kNoPos, kNoTotal, true};
+		else if (fast && sum.seq_min == sum.seq_max)
+			r = uniform_walk(sum, init, acc);
+		else if (fast)
+			r = walk_packet([&](uint32_t i) { return i < nwords ? sm.words[i] : 0u; }, size, init, pp,
+			                [](uint32_t, uint32_t, uint32_t) {});
+		else
+			r = walk_packet([&](uint32_t i) { return i < nwords ? __ldg(pp.data + first + i) : 0u; }, size, init, pp,
+			                [](uint32_t, uint32_t, uint32_t) {});
+		pp.tables[(size_t(p) * 9 + init) * 2 + 0] = r.state | (r.error ? 16u : 0u) | (r.restart << 8);
+		pp.tables[(size_t(p) * 9 + init) * 2 + 1] = r.total;
 	}
 	// The last CTA to finish scans every packet's table (no CTA waits for
 	// another). The tables are the first warp's stores, so its first thread's
@@ -560,7 +560,6 @@ __global__ void __launch_bounds__(kPacketThreads) packet_tables_kernel(const Pac
 		*pp.counter = 0; // ready for the next call
 	scan_packets(pp);
 }
-
 
 __global__ void __launch_bounds__(256) packet_blocks_kernel(const PacketParams pp)
 {
