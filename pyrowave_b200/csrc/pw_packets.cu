@@ -504,7 +504,7 @@ __device__ void scan_packets(const PacketParams &pp)
 	}
 }
 
-__global__ void __launch_bounds__(kPacketThreads) packet_tables_kernel(const PacketParams pp)
+__global__ void __launch_bounds__(kPacketThreads, 2) packet_tables_kernel(const PacketParams pp)
 {
 	extern __shared__ __align__(16) unsigned char s_raw[];
 	PacketSmem &sm = *reinterpret_cast<PacketSmem *>(s_raw);
