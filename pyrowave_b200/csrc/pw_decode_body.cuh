@@ -152,8 +152,8 @@ __device__ __forceinline__ void dequant_block(const BlockReader<kChecked> &rd, c
 		}
 		else
 		{
-			// More than eight planes somewhere in the row (more than sixteen only
-			// in a malformed one): plane by plane.
+			// More than eight planes somewhere in the row, as rows of every frame's LL
+			// blocks have (9 to 12; more than sixteen only a malformed one): plane by plane.
 			uint32_t dec[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 			for (int pl = int(planes) - 1; pl >= 0; pl--)
 			{

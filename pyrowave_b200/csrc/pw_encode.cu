@@ -527,7 +527,7 @@ __device__ __forceinline__ void quant_tile(DwtShared &sh, const LevelParams &p, 
 	const LevelDesc &L = p.L;
 	// Quantise the transmitted bands of this tile: HL, LH, HH (+ LL at the last
 	// level), kGroups bands per round. (A last round on the whole CTA, two warps
-	// per row, repeats the rows' fixed work: 1080p encode 42.25 against 41.4 us.)
+	// per row, repeats the rows' fixed work: 1080p encode 42.25 against 41.0 us.)
 	const int first_band = level == kLevels - 1 ? 0 : 1;
 	const int nb = 4 - first_band;
 	const int grp = threadIdx.x / Split::kGroupThreads, t = threadIdx.x % Split::kGroupThreads;
@@ -537,8 +537,9 @@ __device__ __forceinline__ void quant_tile(DwtShared &sh, const LevelParams &p, 
 		                                  p.band[comp][first_band + bi], tx, ty, buf);
 	__syncthreads();
 	// A half-warp per band finishes its block. Tile dataflow: the resolve waits for
-	// the count of every CTA, released once after all of its bands' rows (a full
-	// fence and count per band cost 4 us of a 4K 4:4:4 frame's encode).
+	// the count of every CTA, released once after all of its bands' rows (with a
+	// full fence and count per band, and one per stored tile, a 4K 4:4:4 frame's
+	// encode took 148.5 instead of 144 us).
 	const int bi = int(threadIdx.x) >> 4;
 	if ((bi & ~1) >= nb)
 		return;
@@ -2196,7 +2197,7 @@ void launch_dwt_forward_level(const LevelParams &p, const PlaneInput &in, const 
 // Two warps per row of 8x8 blocks halve the levels' serial loop, one warp does
 // the row's fixed work once: measured, two are the faster below about two blocks
 // per SM (256x144 encode + decode 39.6 against 40.3 us), one above (720p encode
-// 32.5 -> 32.2 us, 12 mixed frames 853 -> 837 us; 1080p the same).
+// 32.75 -> 32.1 us, 12 mixed frames 857 -> 836 us; 1080p the same).
 constexpr int kSplitRowsBlocks = 2 * 148;
 void launch_quant_pretransformed(const BlockParams &p, const EncodeBuffers &buf, int nblocks, bool programmatic,
                                  cudaStream_t stream)

@@ -419,7 +419,7 @@ __device__ void scan_packets(const PacketParams &pp)
 	for (int p = p0; p < p1; p++)
 		incl = compose(incl, packet_map(pp, p));
 	// The packets of one frame have one map, which changes nothing the second
-	// time: no scan (1080p in 51 packets: 40.3 -> 39.7 us with the decode).
+	// time: no scan (1080p in 51 packets: 40.5 -> 40.1 us with the decode).
 	const unsigned long long one = packet_map(pp, 0);
 	const bool alike = __syncthreads_and(per == 1 && (t >= n || incl == one) && compose(one, one) == one);
 	unsigned long long before = t == 0 ? kIdentityMap : one, all = one;
